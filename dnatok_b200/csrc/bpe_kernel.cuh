@@ -27,8 +27,10 @@
 //   the selection every surviving token is written to its new global position in the other buffer,
 //   re-dealt so that all lanes again own equally many positions.
 //
-// bpe_long_kernel (longer words, one block of 32 warps per word): the same round over arrays in
-//   global memory (tokens in place in the output area, ranks and masks in caller scratch),
+// Longer words are cut into overlapping windows that run bpe_lanes_kernel and are joined exactly (see BpeWindows).
+//
+// bpe_long_kernel (what the windows cannot join, and tables without batched rounds; one block of 32 warps per
+//   word): the same round over arrays in global memory (tokens in place in the output area, ranks and masks in caller scratch),
 //   position-parallel: lane i of a warp handles position 32 g + i and masks come from ballots.
 //
 // Merged tokens (uint16, Hugging Face ids) and per-row counts go to the caller's scratch; the emit
@@ -52,6 +54,9 @@ constexpr int BPE_LONG_CLASS = 6;
 constexpr int BPE_N_CLASSES = BPE_LONG_CLASS + 1;
 constexpr int BPE_LONG_WARPS = 32;
 constexpr int64_t BPE_MAX_POSITIONS = (int64_t)1 << 30;     // longest word of the long class
+constexpr int BPE_WIN = 1024;                   // a window of a long word: what one warp holds ...
+constexpr int BPE_WIN_OVERLAP = 128;            // ... and the positions it shares with the window after it
+constexpr int BPE_WIN_STEP = BPE_WIN - BPE_WIN_OVERLAP;
 
 __host__ __device__ constexpr int bpe_class_capacity(int c) { return (32 * BPE_LANE_SLOTS) << c; }
 // warps per block for teams of W warps
@@ -204,15 +209,19 @@ __device__ __forceinline__ int32_t bpe_put_length(const BpeLengths& L, int64_t r
 
 // One finished row of n tokens into the caller's padded layout, the columns dealt to the T threads that worked on
 // the row (g: this thread's index among them); tok(i) returns token i.
+// i_lo, i_hi: only the columns of tokens [i_lo, i_hi); what precedes the first token and what follows the last
+// one belong to the pieces that hold those.
 template <typename TokFn>
-__device__ __forceinline__ void bpe_write_row(const BpeLengths& L, int64_t row, int n, int g, int T, TokFn tok) {
+__device__ __forceinline__ void bpe_write_row(const BpeLengths& L, int64_t row, int n, int g, int T, TokFn tok, int i_lo = 0,
+                                              int i_hi = INT32_MAX) {
     const int stride = (int)L.out_stride;
     const int kept = n < L.cap_content ? n : (int)L.cap_content;
     const bool has_cls = L.cls_id >= 0, has_sep = L.sep_id >= 0;
     const int total = kept + (has_cls ? 1 : 0) + (has_sep ? 1 : 0);
     const int c0 = (L.pad_left ? stride - total : 0) + (has_cls ? 1 : 0);     // column of the first content token
     const int64_t base = row * L.out_stride;
-    for (int col = g; col < stride; col += T) {
+    const int col_lo = i_lo > 0 ? c0 + i_lo : 0, col_hi = i_hi < n && c0 + i_hi < stride ? c0 + i_hi : stride;
+    for (int col = col_lo + g; col < col_hi; col += T) {
         const int i = col - c0;
         int32_t v = L.pad_id;
         bool on = true;
@@ -361,7 +370,9 @@ __device__ __forceinline__ void bpe_lanes_setup(const BpeLanesShared& sh, const 
 // The words of one list through teams of W warps, in a block of BW warps whose teams each own TEAM_BYTES of
 // the dynamic shared memory.  list == NULL: no binning was done because the caller vouches that every row
 // fits; the n_words rows are taken as they come, and a row longer than direct_limit is flagged and left empty.
-template <int W, int BW, int BAR0, int TEAM_BYTES, bool ST = false>
+// WIN: the words are the windows of long rows (bpe_window_plan_kernel): offsets holds a (start, end) pair per
+// window, window i's tokens go to out_tok + i * BPE_WIN and its count to counts[i] (-1: it did not converge).
+template <int W, int BW, int BAR0, int TEAM_BYTES, bool ST = false, bool WIN = false>
 __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const BpeSmemTable& stab, uint16_t* const sm,
                  const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets,
                  const int32_t* __restrict__ list, const int n_words,
@@ -413,10 +424,11 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             break;
         }
         const int row = list ? list[wi] : wi;
-        const int64_t off = offsets[row];
-        const int64_t n64 = offsets[row + 1] - off;
-        int n = (int)n64;                                    // 1 <= n <= T * P by classification
-        if (!list && (n64 < 1 || n64 > direct_limit)) {      // direct rows are not vetted: an empty row, or one the hint misstated
+        const int64_t oi = WIN ? 2 * (int64_t)wi : (int64_t)row;
+        const int64_t off = offsets[oi];
+        const int64_t n64 = offsets[oi + 1] - off;
+        int n = (int)n64;                                    // 1 <= n <= T * P by classification (windows: by construction)
+        if (!WIN && !list && (n64 < 1 || n64 > direct_limit)) {      // direct rows are not vetted: an empty row, or one the hint misstated
             if (g == 0) {
                 counts[row] = 0;
                 bpe_put_length(len_out, row, 0);
@@ -671,19 +683,22 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             n = n_new; Pp = Pn; inv = inv_n;
         }
 
-        if (len_out.ids) {
+        if (!WIN && len_out.ids) {
             const uint32_t col0 = cur - 2 * g;               // the team's buffer
             bpe_write_row(len_out, row, n, g, T, [&](int q) {
                 const uint32_t l = __umulhi(2u * (uint32_t)q + 1u, inv);
                 return lds_u16(col0 + 2 * (((uint32_t)q - l * Pp) * STRIDE + l));
             });
         } else {
+            uint16_t* const out = out_tok + (WIN ? (int64_t)wi * BPE_WIN : off);
             for (int q = g; q < n; q += T) {
                 const uint32_t l = __umulhi(2u * (uint32_t)q + 1u, inv);
-                out_tok[off + q] = (uint16_t)lds_u16(cur - 2 * g + 2 * (((uint32_t)q - l * Pp) * STRIDE + l));
+                out[q] = (uint16_t)lds_u16(cur - 2 * g + 2 * (((uint32_t)q - l * Pp) * STRIDE + l));
             }
         }
-        if (g == 0) {
+        if (WIN) {
+            if (g == 0) counts[wi] = round >= max_rounds ? -1 : n;
+        } else if (g == 0) {
             counts[row] = n;
             const int32_t bits = bpe_put_length(len_out, row, n) | (round >= max_rounds ? 2 : 0);
             bpe_put_status(status, row, bits, len_out.store_status != 0 && !list);   // binned rows were written by the binning pass
@@ -692,8 +707,8 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
     }
 }
 
-// W: warps per word.
-template <int W>
+// W: warps per word.  WIN: the words are windows of long rows, their number is *list_count.
+template <int W, bool WIN = false>
 __global__ void __launch_bounds__(bpe_block_warps(W) * 32, bpe_min_blocks(W))
 bpe_lanes_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets,
                  const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
@@ -704,16 +719,16 @@ bpe_lanes_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ 
     extern __shared__ uint4 bpe_dyn[];
     BPE_LANES_SHARED(BW, sh);
     bpe_lanes_setup<BW>(sh, t);
-    bpe_lanes_body<W, BW, 1, (int)bpe_team_bytes(W)>(sh, BpeSmemTable{}, reinterpret_cast<uint16_t*>(bpe_dyn), bytes, offsets, list,
-                                                     list ? *list_count : n_direct, work_counter, t, out_tok, counts,
-                                                     status, len_out, direct_limit);
+    bpe_lanes_body<W, BW, 1, (int)bpe_team_bytes(W), false, WIN>(sh, BpeSmemTable{}, reinterpret_cast<uint16_t*>(bpe_dyn), bytes, offsets,
+                                                                 list, WIN || list ? *list_count : n_direct, work_counter, t, out_tok,
+                                                                 counts, status, len_out, direct_limit);
 }
 
 // The same for a vocabulary whose packed table fits into shared memory beside the teams' buffers: one block of
 // 32 warps per SM, the table copied in once per block, every lookup of the general mode answered from it.
 constexpr int BPE_ST_WARPS = 32;
 __host__ __device__ constexpr size_t bpe_st_team_area(int W) { return (size_t)(BPE_ST_WARPS / W) * bpe_team_bytes(W); }
-template <int W>
+template <int W, bool WIN = false>
 __global__ void __launch_bounds__(BPE_ST_WARPS * 32, 1)
 bpe_lanes_st_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets,
                     const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
@@ -735,14 +750,14 @@ bpe_lanes_st_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict
         // A small batch is spread over all blocks: only as many teams of a block take part as the words per
         // block ask for (words are claimed from one counter, and the blocks that start first would otherwise
         // take them all while other SMs stay idle).
-        const int n_words = list ? *list_count : n_direct;
+        const int n_words = WIN || list ? *list_count : n_direct;
         const int active = (n_words + (int)gridDim.x - 1) / (int)gridDim.x;
         if ((int)(threadIdx.x >> 5) / W >= active) return;
     }
     // sixteen teams of two warps need sixteen hardware barriers: barrier 0 is theirs as well once the set-up is over
-    bpe_lanes_body<W, BPE_ST_WARPS, (W == 2 ? 0 : 1), (int)bpe_team_bytes(W), true>(sh, stab, reinterpret_cast<uint16_t*>(bpe_dyn), bytes,
-                                                                     offsets, list, list ? *list_count : n_direct, work_counter,
-                                                                     t, out_tok, counts, status, len_out, direct_limit);
+    bpe_lanes_body<W, BPE_ST_WARPS, (W == 2 ? 0 : 1), (int)bpe_team_bytes(W), true, WIN>(sh, stab, reinterpret_cast<uint16_t*>(bpe_dyn),
+                                                                     bytes, offsets, list, WIN || list ? *list_count : n_direct,
+                                                                     work_counter, t, out_tok, counts, status, len_out, direct_limit);
 }
 
 // Rows of several length classes in one launch: a block of BPE_MIXED_WARPS warps works through the classes
@@ -794,6 +809,214 @@ bpe_mixed_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ 
 #undef BPE_LEVEL
 }
 #undef BPE_SLOTS_DOWN
+
+// Words beyond the lanes kernel's capacity, in windows.  A long word is cut into windows of BPE_WIN positions, each
+// sharing BPE_WIN_OVERLAP positions with the next; the windows are merged like any other short words, one warp or
+// small team each, and joined afterwards at a token that both windows hold at the same place in their overlap.
+//
+// The join is exact.  Take the merges of a word in their order and look at two neighbouring tokens of its result: no
+// merge ever crossed the places where they begin, meet and end, so the merges inside them ran exactly as they run on
+// these two tokens' text alone, which therefore encodes to the same two tokens.  Conversely, if every two neighbours
+// of a sequence of tokens encode to themselves, the sequence is the result for the whole text: before the first merge
+// that crossed one of its borders the merges on either side ran as they run on that pair alone, which would have
+// crossed as well.  (The argument needs no more than the rule itself: lowest rank first, leftmost first.)  Cutting two
+// windows' results at a common token leaves only neighbours that one of the two windows holds.  A border without a
+// common token (a repeat longer than the overlap) sends its word to bpe_long_kernel.
+//
+// One block per word, position-parallel in global memory, left all but a few SMs idle on such batches: 33 words of
+// 40,000 to 400,000 bytes (vocabulary 4,096) took 2,507 us; in windows they take 100 us (merge 75, numbering 8,
+// joins 8, scan 4, copy 5), of which an eighth is work done twice in the overlaps.
+struct BpeWindows {
+    int64_t* span;        // [2 * windows] first byte and end of every window in the batch
+    int32_t* row_of;      // [windows] index of its word in the list of long words
+    int32_t* count;       // [windows] merged tokens
+    int32_t* keep;        // [windows] tokens up to the join with the next window (-1: there is none)
+    int32_t* skip;        // [windows] tokens that the window before holds already
+    int32_t* base;        // [windows] tokens of its word before it
+    int32_t* first;       // [words + 1] first window of every word
+    int32_t* total;       // [words] tokens of the word (-1: left to bpe_long_kernel)
+    uint16_t* tok;        // [windows * BPE_WIN] merged tokens
+};
+
+__device__ __forceinline__ int bpe_window_count(int64_t n) { return (int)((n - BPE_WIN_OVERLAP + BPE_WIN_STEP - 1) / BPE_WIN_STEP); }
+
+// One block: numbers the windows of all long words and writes their spans.
+__global__ void __launch_bounds__(1024)
+bpe_window_plan_kernel(const int64_t* __restrict__ offsets, const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
+                       BpeWindows w, int32_t* __restrict__ n_windows) {
+    __shared__ int32_t s_warp[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_words = *list_count;
+    int carry = 0;
+    for (int i0 = 0; i0 < n_words; i0 += 1024) {
+        const int i = i0 + tid;
+        int nw = 0;
+        if (i < n_words) { const int r = list[i]; nw = bpe_window_count(offsets[r + 1] - offsets[r]); }
+        int x = nw;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(BPE_FULL, x, d);
+            if (lane >= d) x += y;
+        }
+        if (lane == 31) s_warp[warp] = x;
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) { if (k < warp) before += s_warp[k]; all += s_warp[k]; }
+        if (i < n_words) w.first[i] = carry + before + x - nw;
+        carry += all;
+        __syncthreads();
+    }
+    if (tid == 0) { w.first[n_words] = carry; *n_windows = carry; }
+    __syncthreads();
+    for (int i = warp; i < n_words; i += 32) {
+        const int r = list[i], f = w.first[i], nw = w.first[i + 1] - f;
+        const int64_t off = offsets[r], end = offsets[r + 1];
+        for (int k = lane; k < nw; k += 32) {
+            const int64_t a = off + (int64_t)k * BPE_WIN_STEP;
+            w.span[2 * (int64_t)(f + k)] = a;
+            w.span[2 * (int64_t)(f + k) + 1] = a + BPE_WIN < end ? a + BPE_WIN : end;
+            w.row_of[f + k] = i;
+        }
+    }
+}
+
+// One warp per window: where it joins the next window of its word.  tok_len[id]: bytes of a token.
+constexpr int BPE_JOIN_WARPS = 8;
+__global__ void __launch_bounds__(BPE_JOIN_WARPS * 32)
+bpe_window_join_kernel(BpeWindows w, const int32_t* __restrict__ n_windows, const uint16_t* __restrict__ tok_len) {
+    constexpr int OV = BPE_WIN_OVERLAP, PER = OV / 32;
+    __shared__ uint16_t s_id[BPE_JOIN_WARPS][2][OV];          // token that starts at a position of the overlap (0xFFFF: none) ...
+    __shared__ int16_t s_at[BPE_JOIN_WARPS][2][OV];           // ... and its index in its window
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = *n_windows;
+    for (int i = blockIdx.x * BPE_JOIN_WARPS + warp; i < n; i += gridDim.x * BPE_JOIN_WARPS) {
+        const int ca = w.count[i];
+        const bool first = i == 0 || w.row_of[i - 1] != w.row_of[i];
+        const bool last = i + 1 == n || w.row_of[i + 1] != w.row_of[i];
+        if (first && lane == 0) w.skip[i] = 0;
+        if (last) { if (lane == 0) w.keep[i] = ca; continue; }
+        const int cb = w.count[i + 1];
+        const uint16_t* const ta = w.tok + (int64_t)i * BPE_WIN;
+        const uint16_t* const tb = ta + BPE_WIN;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) s_id[warp][0][lane + 32 * k] = s_id[warp][1][lane + 32 * k] = 0xFFFFu;
+        __syncwarp();
+        uint32_t id[2][PER];
+        int len[2][PER], sum[2] = {0, 0};
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int r = PER * lane + k;                     // this window's tokens from its end, the next one's from its start
+            id[0][k] = r < ca ? (uint32_t)ta[ca - 1 - r] : 0xFFFFu;
+            id[1][k] = r < cb ? (uint32_t)tb[r] : 0xFFFFu;
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                len[s][k] = id[s][k] != 0xFFFFu ? (int)__ldg(tok_len + id[s][k]) : OV;
+                sum[s] += len[s][k];
+            }
+        }
+        int at[2] = {sum[0], sum[1]};
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const int y = __shfl_up_sync(BPE_FULL, at[s], d);
+                if (lane >= d) at[s] += y;
+            }
+        at[0] -= sum[0];
+        at[1] -= sum[1];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int r = PER * lane + k;
+            at[0] += len[0][k];                               // bytes from this token's start to the window's end
+            if (at[0] <= OV && id[0][k] != 0xFFFFu) { s_id[warp][0][OV - at[0]] = (uint16_t)id[0][k]; s_at[warp][0][OV - at[0]] = (int16_t)(ca - 1 - r); }
+            if (at[1] < OV && id[1][k] != 0xFFFFu) { s_id[warp][1][at[1]] = (uint16_t)id[1][k]; s_at[warp][1][at[1]] = (int16_t)r; }
+            at[1] += len[1][k];
+        }
+        __syncwarp();
+        int keep = -1, skip = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const int p = lane + 32 * k;
+            const uint32_t a = s_id[warp][0][p];
+            const uint32_t hit = __ballot_sync(BPE_FULL, a != 0xFFFFu && a == s_id[warp][1][p]);
+            if (hit && keep < 0) {
+                const int q = 32 * k + __ffs(hit) - 1;
+                keep = s_at[warp][0][q] + 1;
+                skip = s_at[warp][1][q] + 1;
+            }
+        }
+        if (lane == 0) { w.keep[i] = ca < 0 || cb < 0 ? -1 : keep; w.skip[i + 1] = skip; }
+        __syncwarp();
+    }
+}
+
+// One block per long word: its token count and the place of every window's tokens, or its entry in the list of words
+// that are left to bpe_long_kernel.
+__global__ void __launch_bounds__(1024)
+bpe_window_scan_kernel(const int32_t* __restrict__ list, const int32_t* __restrict__ list_count, BpeWindows w,
+                       int32_t* __restrict__ counts, int32_t* __restrict__ status, BpeLengths len_out,
+                       int32_t* __restrict__ left_list, int32_t* __restrict__ left_count) {
+    __shared__ int32_t s_warp[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_words = *list_count;
+    for (int i = blockIdx.x; i < n_words; i += gridDim.x) {
+        const int f = w.first[i], nw = w.first[i + 1] - f;
+        int carry = 0, bad = 0;
+        for (int k0 = 0; k0 < nw; k0 += 1024) {
+            const int k = k0 + tid;
+            int v = 0;
+            if (k < nw) {
+                const int keep = w.keep[f + k];
+                if (keep < 0) bad = 1;
+                v = keep - w.skip[f + k];
+            }
+            int x = v;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(BPE_FULL, x, d);
+                if (lane >= d) x += y;
+            }
+            if (lane == 31) s_warp[warp] = x;
+            bad = __syncthreads_or(bad);
+            int before = 0, all = 0;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) { if (q < warp) before += s_warp[q]; all += s_warp[q]; }
+            if (k < nw) w.base[f + k] = carry + before + x - v;
+            carry += all;
+            __syncthreads();
+        }
+        if (tid == 0) {
+            const int row = list[i];
+            w.total[i] = bad ? -1 : carry;
+            if (bad) left_list[atomicAdd(left_count, 1)] = row;
+            else {
+                counts[row] = carry;
+                bpe_put_status(status, row, bpe_put_length(len_out, row, carry), false);
+            }
+        }
+    }
+}
+
+// One warp per window: its tokens to their place in the row.
+__global__ void __launch_bounds__(BPE_JOIN_WARPS * 32)
+bpe_window_write_kernel(const int64_t* __restrict__ offsets, const int32_t* __restrict__ list, BpeWindows w,
+                        const int32_t* __restrict__ n_windows, uint16_t* __restrict__ out_tok, BpeLengths len_out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = *n_windows;
+    for (int i = blockIdx.x * BPE_JOIN_WARPS + warp; i < n; i += gridDim.x * BPE_JOIN_WARPS) {
+        const int word = w.row_of[i], total = w.total[word];
+        if (total < 0) continue;
+        const int row = list[word], skip = w.skip[i], m = w.keep[i] - skip, base = w.base[i];
+        const uint16_t* const src = w.tok + (int64_t)i * BPE_WIN + skip;
+        if (len_out.ids) {
+            bpe_write_row(len_out, row, total, lane, 32, [&](int q) { return (uint32_t)src[q - base]; }, base, base + m);
+        } else {
+            uint16_t* const dst = out_tok + offsets[row] + base;
+            for (int q = lane; q < m; q += 32) dst[q] = src[q];
+        }
+    }
+}
 
 // Words beyond the lanes kernel's capacity: one block per word, state in global memory.  The
 // tokens live in place in the output area (uint16 at the input offsets); ranks and the three mask

@@ -130,6 +130,12 @@ int build_bpe_table(const int32_t* a, const int32_t* b, const int32_t* o, int32_
         if (o[r] >= 32) t->hot_ranks = (uint32_t)r;
     t->byte_tok.resize(256);
     for (int i = 0; i < 256; ++i) t->byte_tok[i] = (uint16_t)byte_ids[i];
+    t->tok_len.clear();
+    if (safe) {                               // operands come before what they create
+        t->tok_len.assign(n_tokens, 1);
+        for (int32_t r = 0; r < n; ++r)
+            t->tok_len[o[r]] = (uint16_t)std::min(65535, (int)t->tok_len[a[r]] + (int)t->tok_len[b[r]]);
+    }
     t->n_tokens = n_tokens;
     t->n_merges = (uint32_t)n;
     t->batch_safe = safe;

@@ -25,6 +25,7 @@ struct BpeHostTable {
     uint32_t hot_ranks = 0;            // every rank below this creates an id < 32
     bool bytes_hot = false;            // every initial symbol is an id < 32
     std::vector<uint16_t> byte_tok;    // [256] initial symbol of each byte
+    std::vector<uint16_t> tok_len;     // [n_tokens] bytes a token stands for, at most 65,535; empty when the table is not batch-safe
     // The same table packed for a kernel that keeps it in shared memory (empty when an id or a displacement does
     // not fit 16 bits): 16-bit displacements [n_tokens + 1], then 32-bit slots (left id << 16) | rank up to the last
     // used one plus one empty slot (larger indices are clamped to it), then one word per rank,

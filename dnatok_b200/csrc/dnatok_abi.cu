@@ -85,6 +85,7 @@ struct DeviceTables {
     uint16_t* merge_out = nullptr;
     uint64_t* hot = nullptr;
     uint16_t* byte_tok = nullptr;
+    uint16_t* tok_len = nullptr;     // BPE: bytes per token (when the table is batch-safe)
     int sm_count = 0;
     // host-pipeline staging (grow only)
     uint8_t* st_bytes = nullptr;  size_t st_bytes_cap = 0;
@@ -153,7 +154,7 @@ int tables_for_current_device(dnatok_handle* h, DeviceTables** out) {
             ~Undo() {
                 if (keep) return;
                 DeviceTables& x = h->dev[dev];
-                void* ptrs[] = {x.lut256, x.start_lut, x.kmer_ids, x.table5, x.exp_off, x.exp_ids, x.disp, x.slots, x.merge_out, x.hot, x.byte_tok, x.bpe_compact};
+                void* ptrs[] = {x.lut256, x.start_lut, x.kmer_ids, x.table5, x.exp_off, x.exp_ids, x.disp, x.slots, x.merge_out, x.hot, x.byte_tok, x.tok_len, x.bpe_compact};
                 for (void* p : ptrs) if (p) cudaFree(p);
                 h->dev.erase(dev);
             }
@@ -175,6 +176,7 @@ int tables_for_current_device(dnatok_handle* h, DeviceTables** out) {
             if ((rc = upload(&d.merge_out, h->bpe.merge_out))) return rc;
             if ((rc = upload(&d.hot, h->bpe.hot))) return rc;
             if ((rc = upload(&d.byte_tok, h->bpe.byte_tok))) return rc;
+            if (!h->bpe.tok_len.empty() && (rc = upload(&d.tok_len, h->bpe.tok_len))) return rc;
             const BpeLaunchInfo* info;
             if ((rc = bpe_launch_info(dev, &info))) return rc;     // configures every merge kernel once per device
         }
@@ -264,6 +266,8 @@ BpeScratch bpe_scratch_layout(const dnatok_handle* h, void* base, int64_t n_rows
 // shared-memory attribute, so a later launch does nothing but launch.
 struct BpeLaunchInfo { int lanes[BPE_LONG_CLASS]; int mixed; int st_room[BPE_LONG_CLASS]; };   // resident blocks per SM of every merge kernel; st_room: bytes a shared-memory table may take beside the teams of each width (0: kernel not usable)
 
+constexpr int BPE_WIN_MAX_TEAM = 8;   // widest team that works on a window of a long word (four positions per lane)
+
 template <int W>
 int bpe_setup_st(int* room) {
     cudaFuncAttributes fa;
@@ -275,6 +279,8 @@ int bpe_setup_st(int* room) {
     *room = 0;
     if (dyn <= (int64_t)bpe_st_team_area(W)) return 0;
     CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_st_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    if constexpr (W <= BPE_WIN_MAX_TEAM)
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_st_kernel<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     *room = (int)(dyn - (int64_t)bpe_st_team_area(W));
     return 0;
 }
@@ -284,6 +290,8 @@ int bpe_setup_lanes(int* bps) {
     constexpr int BW = bpe_block_warps(W);
     const size_t smem = (size_t)(BW / W) * bpe_team_bytes(W);
     CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if constexpr (W <= BPE_WIN_MAX_TEAM)
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_kernel<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, bpe_lanes_kernel<W>, BW * 32, smem));
     if (*bps < 1) *bps = 1;
     return 0;
@@ -311,6 +319,10 @@ int bpe_launch_info(int dev, const BpeLaunchInfo** out) {
         cudaFuncAttributes fa;
         CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_long_kernel));      // loads the kernel's code now, not at its first launch
         CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_classify_kernel));
+        CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_plan_kernel));
+        CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_join_kernel));
+        CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_scan_kernel));
+        CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_write_kernel));
         // ... and the kernels of the output stage, for both id widths
         CUDA_TRY(cudaFuncGetAttributes(&fa, span_lengths_kernel));
         CUDA_TRY(cudaFuncGetAttributes(&fa, scan_lengths_kernel));
@@ -408,6 +420,77 @@ int bpe_team_width(const DeviceTables& d, const BpeLaunchInfo& li, int64_t n_row
     return w;
 }
 
+// Where the windows of the long words live: in the long class's working area, which bpe_long_kernel uses for the words
+// the windows leave to it, after all other words are done.  Their list sits at the area's end, which bpe_long_kernel
+// never reaches (it takes at most 2.375 of the area's 2.5 bytes per byte).  Returns false when the area is too small.
+bool bpe_window_layout(const BpeScratch& s, int64_t n_rows, int64_t total_bytes, BpeWindows* w, int32_t** left_list, int64_t* most_windows) {
+    int64_t words = total_bytes / (bpe_class_capacity(BPE_LONG_CLASS - 1) + 1);      // long words the batch can hold
+    if (words > n_rows) words = n_rows;
+    const int64_t wins = total_bytes / BPE_WIN_STEP + words;
+    size_t o = 0;
+    uint8_t* b = s.long_area;
+    auto take = [&](size_t bytes) { uint8_t* p = b + o; o += align_up(bytes, 16); return p; };
+    w->tok = (uint16_t*)take((size_t)wins * BPE_WIN * 2);
+    w->span = (int64_t*)take((size_t)wins * 16);
+    for (int32_t** p : {&w->row_of, &w->count, &w->keep, &w->skip, &w->base}) *p = (int32_t*)take((size_t)wins * 4);
+    w->first = (int32_t*)take((size_t)(words + 1) * 4);
+    w->total = (int32_t*)take((size_t)words * 4);
+    const size_t list_bytes = align_up((size_t)words * 4, 16);
+    *left_list = (int32_t*)(b + s.long_bytes - list_bytes);
+    *most_windows = wins;
+    return words > 0 && wins < INT32_MAX && o + list_bytes <= s.long_bytes;
+}
+
+template <int W>
+int launch_bpe_windows(const DeviceTables& d, const BpeLaunchInfo& li, const BpeDeviceTable& t, const uint8_t* bytes, const BpeWindows& w,
+                       int64_t most_windows, const int32_t* n_windows, int32_t* work, cudaStream_t st) {
+    constexpr int WI = W == 1 ? 0 : W == 2 ? 1 : W == 4 ? 2 : 3;
+    const BpeLengths none{};
+    if (t.compact && g_bpe_smem_table.load() && t.compact_bytes <= (uint32_t)li.st_room[WI]) {
+        const unsigned grid = (unsigned)(most_windows < d.sm_count ? most_windows : d.sm_count);
+        bpe_lanes_st_kernel<W, true><<<grid, BPE_ST_WARPS * 32, bpe_st_team_area(W) + t.compact_bytes, st>>>(
+            bytes, w.span, nullptr, n_windows, work, t, w.tok, w.count, nullptr, none, 0, 0);
+        LAUNCH_CHECK("bpe_lanes_st_kernel (windows)");
+        return 0;
+    }
+    constexpr int BW = bpe_block_warps(W), TEAMS = BW / W;
+    const int64_t need = (most_windows + TEAMS - 1) / TEAMS, resident = (int64_t)d.sm_count * li.lanes[WI];
+    bpe_lanes_kernel<W, true><<<(unsigned)(need < resident ? need : resident), BW * 32, (size_t)TEAMS * bpe_team_bytes(W), st>>>(
+        bytes, w.span, nullptr, n_windows, work, t, w.tok, w.count, nullptr, none, 0, 0);
+    LAUNCH_CHECK("bpe_lanes_kernel (windows)");
+    return 0;
+}
+
+// The long words of a batch in windows; the words whose windows do not join are left in left_list / left_count.
+int run_bpe_windows(const DeviceTables& d, const BpeLaunchInfo& li, const BpeDeviceTable& t, const uint8_t* bytes, const int64_t* offsets,
+                    int64_t n_rows, const BpeScratch& s, const BpeWindows& w, int64_t most_windows, int32_t* left_list, int32_t* status,
+                    const BpeLengths& lo, cudaStream_t st) {
+    // counters behind those of the length classes, zeroed with them
+    int32_t* const n_windows = s.class_count + BPE_N_CLASSES;
+    int32_t* const left_count = n_windows + 1;
+    int32_t* const work = s.work + BPE_N_CLASSES;
+    const int32_t* const list = s.class_list + (int64_t)BPE_LONG_CLASS * n_rows;
+    const int32_t* const list_count = s.class_count + BPE_LONG_CLASS;
+    bpe_window_plan_kernel<<<1, 1024, 0, st>>>(offsets, list, list_count, w, n_windows);
+    LAUNCH_CHECK("bpe_window_plan_kernel");
+    const int width = bpe_team_width(d, li, most_windows, BPE_WIN);
+    int rc = width >= 8 ? launch_bpe_windows<8>(d, li, t, bytes, w, most_windows, n_windows, work, st)
+           : width >= 4 ? launch_bpe_windows<4>(d, li, t, bytes, w, most_windows, n_windows, work, st)
+           : width >= 2 ? launch_bpe_windows<2>(d, li, t, bytes, w, most_windows, n_windows, work, st)
+                        : launch_bpe_windows<1>(d, li, t, bytes, w, most_windows, n_windows, work, st);
+    if (rc) return rc;
+    const int64_t need = (most_windows + BPE_JOIN_WARPS - 1) / BPE_JOIN_WARPS, most = (int64_t)d.sm_count * 8;
+    const unsigned grid = (unsigned)(need < most ? need : most);
+    bpe_window_join_kernel<<<grid, BPE_JOIN_WARPS * 32, 0, st>>>(w, n_windows, d.tok_len);
+    LAUNCH_CHECK("bpe_window_join_kernel");
+    const unsigned word_grid = (unsigned)(n_rows < (int64_t)d.sm_count * 2 ? n_rows : (int64_t)d.sm_count * 2);
+    bpe_window_scan_kernel<<<word_grid, 1024, 0, st>>>(list, list_count, w, s.counts, status, lo, left_list, left_count);
+    LAUNCH_CHECK("bpe_window_scan_kernel");
+    bpe_window_write_kernel<<<grid, BPE_JOIN_WARPS * 32, 0, st>>>(offsets, list, w, n_windows, s.tokens, lo);
+    LAUNCH_CHECK("bpe_window_write_kernel");
+    return 0;
+}
+
 // lengths (may be NULL) receives every row's final token count for the format rf.
 // ids (may be NULL): when given and the layout is padded, the merge kernels write the final ids and mask
 // themselves and no output pass is needed afterwards.
@@ -463,9 +546,22 @@ int run_bpe_merge(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes,
         if (grid > n_rows) grid = n_rows;
         if (grid > d.sm_count) grid = d.sm_count;
         if (grid < 1) grid = 1;
+        const int32_t* long_list = s.class_list + (int64_t)BPE_LONG_CLASS * n_rows;
+        const int32_t* long_count = s.class_count + BPE_LONG_CLASS;
+        // In windows where a long word is known to be there: the caller's bounds say so, or the rows are half as long on
+        // average.  Otherwise (no bounds, ordinary rows) five more launches that find nothing to do would cost every
+        // such batch about 10 us.
+        BpeWindows w;
+        int32_t* left_list;
+        int64_t most_windows;
+        if (d.tok_len && (h->hint_max_row > 0 || total_bytes / n_rows > bpe_class_capacity(BPE_LONG_CLASS - 1) / 2) &&
+            bpe_window_layout(s, n_rows, total_bytes, &w, &left_list, &most_windows)) {
+            if (int rc = run_bpe_windows(d, *li, t, bytes, offsets, n_rows, s, w, most_windows, left_list, status, lo, st)) return rc;
+            long_list = left_list;
+            long_count = s.class_count + BPE_N_CLASSES + 1;
+        }
         bpe_long_kernel<<<(unsigned)grid, BPE_LONG_WARPS * 32, 0, st>>>(
-            bytes, offsets, s.class_list + (int64_t)BPE_LONG_CLASS * n_rows, s.class_count + BPE_LONG_CLASS,
-            s.work + BPE_LONG_CLASS, t, s.tokens, s.counts, status, s.long_area, s.long_cursor, lo);
+            bytes, offsets, long_list, long_count, s.work + BPE_LONG_CLASS, t, s.tokens, s.counts, status, s.long_area, s.long_cursor, lo);
         LAUNCH_CHECK("bpe_long_kernel");
     }
     int rc;
@@ -1062,7 +1158,7 @@ void dnatok_destroy(dnatok_handle* h) {
         DeviceTables& d = kv.second;
         if (cudaSetDevice(kv.first) != cudaSuccess) continue;
         if (d.stream) cudaStreamSynchronize(d.stream);
-        void* ptrs[] = {d.lut256, d.start_lut, d.table5, d.exp_off, d.exp_ids, d.kmer_ids, d.disp, d.slots, d.merge_out, d.hot, d.byte_tok, d.bpe_compact, d.st_bytes, d.st_offsets,
+        void* ptrs[] = {d.lut256, d.start_lut, d.table5, d.exp_off, d.exp_ids, d.kmer_ids, d.disp, d.slots, d.merge_out, d.hot, d.byte_tok, d.tok_len, d.bpe_compact, d.st_bytes, d.st_offsets,
                         d.st_ids, d.st_mask, d.st_lengths, d.st_status, d.st_out_offsets, d.st_scratch};
         for (void* p : ptrs) if (p) cudaFree(p);
         if (d.stream) cudaStreamDestroy(d.stream);
