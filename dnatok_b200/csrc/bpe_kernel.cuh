@@ -137,7 +137,9 @@ struct ChainPrep {
     bool fast;
 };
 
-template <bool DOWN>
+// L: lanes of a segment; the lanes of a warp form 32 / L segments whose words are separate (L < 32: `lane` is the lane
+// within its segment, and nothing enters a segment).
+template <bool DOWN, int L = 32>
 __device__ __forceinline__ ChainPrep chain_prepare(uint32_t c, int top, uint32_t full, int lane, uint32_t& block_fn) {
     ChainPrep p;
     p.odd0 = run_parity(c);
@@ -146,34 +148,34 @@ __device__ __forceinline__ ChainPrep chain_prepare(uint32_t c, int top, uint32_t
     p.fast = __ballot_sync(BPE_FULL, c == full) == 0u;
     if (p.fast) {
         p.f = out0;
-        block_fn = __shfl_sync(BPE_FULL, out0, DOWN ? 0 : 31) * 3u;      // a constant function
+        if (L == 32) block_fn = __shfl_sync(BPE_FULL, out0, DOWN ? 0 : 31) * 3u;      // a constant function
     } else {
         uint32_t f = out0 | ((((p.odd0 ^ p.fr) >> top) & 1u) << 1);
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t other = DOWN ? __shfl_down_sync(BPE_FULL, f, d) : __shfl_up_sync(BPE_FULL, f, d);
-            if (DOWN ? lane + d < 32 : lane >= d) f = carry_then(other, f);     // the lanes before this one apply first
+        for (int d = 1; d < L; d <<= 1) {
+            const uint32_t other = DOWN ? __shfl_down_sync(BPE_FULL, f, d, L) : __shfl_up_sync(BPE_FULL, f, d, L);
+            if (DOWN ? lane + d < L : lane >= d) f = carry_then(other, f);     // the lanes before this one apply first
         }
         p.f = f;
-        block_fn = __shfl_sync(BPE_FULL, f, DOWN ? 0 : 31);
+        if (L == 32) block_fn = __shfl_sync(BPE_FULL, f, DOWN ? 0 : 31);
     }
     return p;
 }
 
-template <bool DOWN>
+template <bool DOWN, int L = 32>
 __device__ __forceinline__ uint32_t chain_finish(const ChainPrep& p, bool carry, int lane) {
-    const uint32_t before = DOWN ? __shfl_down_sync(BPE_FULL, p.f, 1) : __shfl_up_sync(BPE_FULL, p.f, 1);
-    const bool cin = (DOWN ? lane == 31 : lane == 0) ? carry : (p.fast ? before != 0u : carry_apply(before, carry) != 0u);
+    const uint32_t before = DOWN ? __shfl_down_sync(BPE_FULL, p.f, 1, L) : __shfl_up_sync(BPE_FULL, p.f, 1, L);
+    const bool cin = (DOWN ? lane == L - 1 : lane == 0) ? carry : (p.fast ? before != 0u : carry_apply(before, carry) != 0u);
     return cin ? p.odd0 ^ p.fr : p.odd0;
 }
 
 // Both steps for blocks visited one after the other: `carry` enters the block and leaves it updated.
-template <bool DOWN>
+template <bool DOWN, int L = 32>
 __device__ __forceinline__ uint32_t chain_parity(uint32_t c, int top, uint32_t full, bool& carry, int lane) {
-    uint32_t fn;
-    const ChainPrep p = chain_prepare<DOWN>(c, top, full, lane, fn);
-    const uint32_t odd = chain_finish<DOWN>(p, carry, lane);
-    carry = carry_apply(fn, carry) != 0u;
+    uint32_t fn = 0;
+    const ChainPrep p = chain_prepare<DOWN, L>(c, top, full, lane, fn);
+    const uint32_t odd = chain_finish<DOWN, L>(p, carry, lane);
+    if (L == 32) carry = carry_apply(fn, carry) != 0u;
     return odd;
 }
 
@@ -243,10 +245,15 @@ __device__ __forceinline__ void bpe_write_row(const BpeLengths& L, int64_t row, 
 // Bin rows by length: class_count[c] rows land in class_list[c * n_rows ...].  One atomic per
 // warp and class (rows of a batch mostly share a class).  Classes outside class_mask are not
 // launched by the host; a row that belongs to one is flagged instead of being dropped silently.
+// short_bins: rows of the first class that fit a half, a quarter or an eighth of a warp are listed apart, k-th bin
+// (1 << k rows per warp) with its counter at class_count[BPE_SHORT_COUNT + k] and its list backwards from the end of
+// class k's, which it cannot meet: a row is in one list only.
+constexpr int BPE_SHORT_BINS = 3;
+constexpr int BPE_SHORT_COUNT = BPE_N_CLASSES + 1;            // after the counters of the windows; bins count from 1
 __global__ void bpe_classify_kernel(const int64_t* __restrict__ offsets, int64_t n_rows,
                                     int32_t* __restrict__ class_count, int32_t* __restrict__ class_list,
                                     int32_t* __restrict__ counts, int32_t* __restrict__ status,
-                                    uint32_t class_mask, BpeLengths len_out) {
+                                    uint32_t class_mask, BpeLengths len_out, bool short_bins) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     int c = -1;
@@ -259,6 +266,9 @@ __global__ void bpe_classify_kernel(const int64_t* __restrict__ offsets, int64_t
             while (c < BPE_LONG_CLASS && (int64_t)bpe_class_capacity(c) < n) ++c;
             if (n > BPE_MAX_POSITIONS) { bits = 1; c = -1; }
             else if (!((class_mask >> c) & 1u)) { bits = 8; c = -1; }   // outside the caller's length hint
+            else if (short_bins)
+                for (int k = BPE_SHORT_BINS; k >= 1 && c == 0; --k)
+                    if (n <= (bpe_class_capacity(0) >> k)) c = BPE_SHORT_COUNT + k;
         }
         if (c < 0) {                                              // no kernel will visit this row
             bpe_put_length(len_out, i, 0);
@@ -266,14 +276,16 @@ __global__ void bpe_classify_kernel(const int64_t* __restrict__ offsets, int64_t
         }
         bpe_put_status(status, i, bits, len_out.store_status != 0);
     }
-    for (int k = 0; k < BPE_N_CLASSES; ++k) {
+    const int n_lists = short_bins ? BPE_SHORT_COUNT + BPE_SHORT_BINS + 1 : BPE_N_CLASSES;
+    for (int k = 0; k < n_lists; ++k) {
         const uint32_t m = __ballot_sync(0xffffffffu, c == k);
         if (m == 0) continue;
         const int leader = __ffs(m) - 1;
         int base = 0;
         if (lane == leader) base = atomicAdd(class_count + k, __popc(m));
         base = __shfl_sync(0xffffffffu, base, leader);
-        if (c == k) class_list[(int64_t)k * n_rows + base + __popc(m & ((1u << lane) - 1u))] = (int32_t)i;
+        const int at = base + __popc(m & ((1u << lane) - 1u));
+        if (c == k) class_list[k < BPE_N_CLASSES ? (int64_t)k * n_rows + at : (int64_t)(k - BPE_SHORT_COUNT + 1) * n_rows - 1 - at] = (int32_t)i;
     }
 }
 
@@ -372,7 +384,9 @@ __device__ __forceinline__ void bpe_lanes_setup(const BpeLanesShared& sh, const 
 // fits; the n_words rows are taken as they come, and a row longer than direct_limit is flagged and left empty.
 // WIN: the words are the windows of long rows (bpe_window_plan_kernel): offsets holds a (start, end) pair per
 // window, window i's tokens go to out_tok + i * BPE_WIN and its count to counts[i] (-1: it did not converge).
-template <int W, int BW, int BAR0, int TEAM_BYTES, bool ST = false, bool WIN = false>
+// G (one warp per team only): words a warp works on at once, 32 / G lanes each.  A round's work outside the slots (scans,
+// votes, walk parities) costs a warp the same whatever the word's length, so short words share it.
+template <int W, int BW, int BAR0, int TEAM_BYTES, bool ST = false, bool WIN = false, int G = 1>
 __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const BpeSmemTable& stab, uint16_t* const sm,
                  const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets,
                  const int32_t* __restrict__ list, const int n_words,
@@ -380,8 +394,10 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
                  uint16_t* __restrict__ out_tok, int32_t* __restrict__ counts,
                  int32_t* __restrict__ status, const BpeLengths& len_out, int32_t direct_limit) {
     constexpr int P = BPE_LANE_SLOTS;
-    constexpr int T = 32 * W;                    // lanes of a team
-    constexpr int STRIDE = T + 2;                // elements between the slots of one lane
+    static_assert(G == 1 || (W == 1 && !WIN), "only single warps share words");
+    constexpr int T = 32 * W / G;                // lanes of a word
+    constexpr int L = 32 / G;                    // ... and of them in one warp
+    constexpr int STRIDE = 32 * W + 2;           // elements between the slots of one lane
     constexpr int BUF = (P + 1) * STRIDE;        // one token buffer: P slots and the copy of the next lane's first token
     static_assert(TEAM_BYTES >= (int)bpe_team_bytes(W), "team area too small");
     uint16_t* const s_btok = sh.btok;
@@ -392,12 +408,13 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int team = warp / W, tw = warp % W;    // team, warp within team
     int32_t* const s_word = sh.word + team * W;
-    const int g = tw * 32 + lane;                // lane within team
+    const int g = G > 1 ? lane % L : tw * 32 + lane;   // lane within the word's lanes
+    const int part = lane / L;                   // which of the warp's words (G > 1)
     // All token traffic goes through shared-memory byte addresses held in registers.
     constexpr uint32_t S2 = 2 * STRIDE;          // bytes between the slots of one lane
     const uint32_t team_base = (uint32_t)team * (TEAM_BYTES / 2);
     const uint32_t hot_base = smem_u32(sh.hot);
-    uint32_t cur = smem_u32(sm + team_base + g); // this lane's column in the buffer of live tokens
+    uint32_t cur = smem_u32(sm + team_base + (G > 1 ? lane : g)); // this lane's column in the buffer of live tokens
     uint32_t nxt = cur + 2 * BUF;                // ... and in the buffer the round writes
     uint32_t* const xf = reinterpret_cast<uint32_t*>(sm + team_base + 2 * BUF);   // [T] entry of every lane's first pair (W > 1)
     uint32_t* const xl = xf + T;                                                  // [T] entry of every lane's last pair  (W > 1)
@@ -408,8 +425,12 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
     for (;;) {
         int wi;
         if (!work_counter) {
-            wi = first ? (int)blockIdx.x + (int)gridDim.x * team : n_words;
+            wi = first ? (int)blockIdx.x + (int)gridDim.x * (team * G + (G > 1 ? part : 0)) : n_words;
             first = false;
+        } else if (G > 1) {
+            wi = 0;
+            if (lane == 0) wi = atomicAdd(work_counter, G);
+            wi = __shfl_sync(BPE_FULL, wi, 0) + part;
         } else if (W == 1) {
             wi = 0;
             if (lane == 0) wi = atomicAdd(work_counter, 1);
@@ -419,16 +440,18 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             team_sync<W, BW, BAR0>(team);
             wi = s_word[0];
         }
-        if (wi >= n_words) {
+        if (G > 1 ? !__any_sync(BPE_FULL, wi < n_words) : wi >= n_words) {
             team_sync<W, BW, BAR0>(team);                    // the claim slot is reused by whatever this team runs next
             break;
         }
-        const int row = list ? list[wi] : wi;
+        const bool here = G == 1 || wi < n_words;            // the last words may not fill a warp
+        const int row = !here ? 0 : !list ? wi : G > 1 ? list[-wi] : list[wi];    // short rows are listed backwards (bpe_classify_kernel)
         const int64_t oi = WIN ? 2 * (int64_t)wi : (int64_t)row;
         const int64_t off = offsets[oi];
-        const int64_t n64 = offsets[oi + 1] - off;
+        const int64_t n64 = here ? offsets[oi + 1] - off : 0;
         int n = (int)n64;                                    // 1 <= n <= T * P by classification (windows: by construction)
-        if (!WIN && !list && (n64 < 1 || n64 > direct_limit)) {      // direct rows are not vetted: an empty row, or one the hint misstated
+        if (G > 1 && !list && n64 > direct_limit) n = 0;     // flagged at the end
+        if (G == 1 && !WIN && !list && (n64 < 1 || n64 > direct_limit)) {      // direct rows are not vetted: an empty row, or one the hint misstated
             if (g == 0) {
                 counts[row] = 0;
                 bpe_put_length(len_out, row, 0);
@@ -439,6 +462,7 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             continue;
         }
         uint32_t Pp = (uint32_t)(n + T - 1) / T;             // positions per lane: lane g owns [g Pp, (g + 1) Pp)
+        if (G > 1) Pp = max(__reduce_max_sync(BPE_FULL, Pp), 1u);   // the same for all words of the warp
         uint32_t inv = s_inv[Pp];
 
         // While every token of the word is a small id (all_hot) the pairs come from the shared-memory
@@ -446,7 +470,7 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
         // come from the table in global memory and the filler is the id one past the vocabulary.
         bool all_hot = t.bytes_hot != 0u;
         uint32_t filler = all_hot ? BPE_FILLER : t.filler;
-        if (g == 0) sts_u16(cur + 2 * T, filler);            // what the last lane sees as "the next lane's first token"
+        if (G == 1 && g == 0) sts_u16(cur + 2 * T, filler);  // what the last lane sees as "the next lane's first token"
         // Every lane fetches its own chunk of the word as aligned 32-bit words (all requested before the
         // first is used), maps the bytes to tokens and fills its column.
         {
@@ -458,7 +482,7 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             uint32_t w[P / 4 + 1];
 #pragma unroll
             for (int k = 0; k <= P / 4; ++k)                 // a word is read when it holds a byte of the word
-                w[k] = (4 * k < (int)(Pp + mis) && first + 4 * k < n && first + 4 * k + 3 >= 0) ? __ldg(src + k) : 0u;
+                w[k] = (4 * k < (int)(Pp + mis) && first + 4 * k < n && first + 4 * k + 3 >= 0 && (G == 1 || n > 0)) ? __ldg(src + k) : 0u;
 #pragma unroll
             for (int k = 0; k < P / 4; ++k) {
                 if (4 * k < (int)Pp) {
@@ -474,14 +498,12 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
         team_sync<W, BW, BAR0>(team);
 
         int round = 0;
-        const int max_rounds = n + 2;
+        const int max_rounds = (G > 1 ? __reduce_max_sync(BPE_FULL, n) : n) + 2;
         for (; round < max_rounds; ++round) {
             const int top = (int)Pp - 1, sh = 32 - (int)Pp;
             const int p0 = g * (int)Pp;
-            // the next lane's first token becomes this lane's slot Pp, so that every slot finds its right neighbour one slot up
-            uint32_t t_up = lds_u16(cur + 2);                // handed from slot to slot: the token one slot up
-            sts_u16(cur + Pp * S2, t_up);
-            team_sync<W, BW, BAR0>(team);
+            uint32_t t_up = lds_u16(cur + 2);                // the next lane's first token; then handed from slot to slot: the token one slot up
+            if (G > 1 && g == L - 1) t_up = filler;
 
             // ---- A: entries of the lane's pairs, the word's bound, "right neighbour ranks better" bits.
             // While every token of the word is a small id all pairs come from the shared-memory table and
@@ -530,13 +552,17 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             }
             gt &= (1u << top) - 1u;                          // the last slot was compared with nothing; set below
             const uint32_t v_first = val[0];
-            emin = __reduce_min_sync(BPE_FULL, emin);
+            if (G == 1) emin = __reduce_min_sync(BPE_FULL, emin);
+            else {
+#pragma unroll
+                for (int d = 1; d < L; d <<= 1) emin = min(emin, __shfl_xor_sync(BPE_FULL, emin, d));
+            }
             uint32_t v_nf, v_pl;                             // the next lane's first entry, the previous lane's last entry
             if (W == 1) {
-                v_nf = __shfl_down_sync(BPE_FULL, v_first, 1);
-                v_pl = __shfl_up_sync(BPE_FULL, v_top, 1);
-                if (lane == 31) v_nf = BPE_FULL;
-                if (lane == 0) v_pl = BPE_FULL;
+                v_nf = __shfl_down_sync(BPE_FULL, v_first, 1, L);
+                v_pl = __shfl_up_sync(BPE_FULL, v_top, 1, L);
+                if (g == L - 1) v_nf = BPE_FULL;
+                if (g == 0) v_pl = BPE_FULL;
             } else {
                 xf[g] = v_first;
                 xl[g] = v_top;
@@ -547,7 +573,8 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
                 v_nf = g + 1 < T ? xf[g + 1] : BPE_FULL;
                 v_pl = g > 0 ? xl[g - 1] : BPE_FULL;
             }
-            if (emin == BPE_FULL) break;                     // no pair can merge: done (uniform over the team)
+            // no pair can merge: done (uniform over the team; words that share a warp wait for the last one, unchanged)
+            if (G > 1 ? __all_sync(BPE_FULL, emin == BPE_FULL) : emin == BPE_FULL) break;
             const uint32_t Bs = emin & 0xFFFF0000u;          // rank < B  <=>  entry < B << 16
 
             // ---- B: candidate and link masks of the lane's positions
@@ -574,26 +601,27 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             if (W == 1) {
                 all_hot = all_hot && !__any_sync(BPE_FULL, big);
                 bool carry = false;
-                const uint32_t odd_r = __brev(chain_parity<true>(__brev(link_r) >> sh, top, full, carry, lane) << sh);
+                const uint32_t odd_r = __brev(chain_parity<true, L>(__brev(link_r) >> sh, top, full, carry, g) << sh);
                 carry = false;
-                const uint32_t odd_l = chain_parity<false>(link_l, top, full, carry, lane);
+                const uint32_t odd_l = chain_parity<false, L>(link_l, top, full, carry, g);
                 sel = cand & ~odd_l & ~odd_r;
                 if (t.single_step) {                         // only the leftmost pair of the lowest rank
-                    const uint32_t any = __ballot_sync(BPE_FULL, sel != 0u);
-                    sel = lane == __ffs(any) - 1 ? (sel & (0u - sel)) : 0u;
+                    uint32_t any = __ballot_sync(BPE_FULL, sel != 0u);
+                    if (G > 1) any = (any >> (part * L)) & (BPE_FULL >> (32 - L));
+                    sel = g == __ffs(any) - 1 ? (sel & (0u - sel)) : 0u;
                 }
-                uint32_t prev = __shfl_up_sync(BPE_FULL, sel >> top, 1);
-                if (lane == 0) prev = 0u;
+                uint32_t prev = __shfl_up_sync(BPE_FULL, sel >> top, 1, L);
+                if (g == 0) prev = 0u;
                 kept = valid & ~((sel << 1) | prev);
                 const int x = __popc(kept);
                 int incl = x;
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int y = __shfl_up_sync(BPE_FULL, incl, d);
-                    if (lane >= d) incl += y;
+                for (int d = 1; d < L; d <<= 1) {
+                    const int y = __shfl_up_sync(BPE_FULL, incl, d, L);
+                    if (g >= d) incl += y;
                 }
                 q0 = incl - x;
-                n_new = __shfl_sync(BPE_FULL, incl, 31);
+                n_new = __shfl_sync(BPE_FULL, incl, L - 1, L);
             } else {
                 // every warp works on its own 32 lanes; what crosses warps are the blocks' carry functions
                 // (first barrier) and their survivor counts with the border bits (second barrier)
@@ -652,7 +680,9 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
 
             // ---- C: merge, and deal the survivors out again in the other buffer, last slot first.
             // Position q goes to lane l = q / Pn, slot q - l Pn: byte 2 (q STRIDE - l (Pn STRIDE - 1)) of the buffer.
-            const uint32_t Pn = (uint32_t)(n_new + T - 1) / T, inv_n = s_inv[Pn];
+            uint32_t Pn = (uint32_t)(n_new + T - 1) / T;
+            if (G > 1) Pn = __reduce_max_sync(BPE_FULL, Pn);
+            const uint32_t inv_n = s_inv[Pn];
             const uint32_t back = 2 * (Pn * STRIDE - 1);
             const uint32_t dst = nxt - 2 * g;                // start of the buffer the round writes
             uint32_t q = (uint32_t)q0 + (uint32_t)__popc(kept);
@@ -671,12 +701,12 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
             }
             {                                                // filler behind the new end, up to the lanes' common slot count
                 filler = all_hot ? BPE_FILLER : t.filler;
-                const uint32_t pt = (uint32_t)n_new + (uint32_t)g;
-                if (pt < Pn * T) {
+                for (uint32_t pt = (uint32_t)n_new + (uint32_t)g; pt < Pn * T; pt += T) {    // one trip unless words share the warp
                     const uint32_t l_ = __umulhi(2u * pt + 1u, inv_n);
                     sts_u16(dst + pt * S2 - l_ * back, filler);
+                    if (G == 1) break;
                 }
-                if (g == 0) sts_u16(dst + 2 * T, filler);    // the column behind the last lane
+                if (G == 1 && g == 0) sts_u16(dst + 2 * T, filler);    // the column behind the last lane
             }
             team_sync<W, BW, BAR0>(team);
             const uint32_t sw = cur; cur = nxt; nxt = sw;
@@ -685,7 +715,7 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
 
         if (!WIN && len_out.ids) {
             const uint32_t col0 = cur - 2 * g;               // the team's buffer
-            bpe_write_row(len_out, row, n, g, T, [&](int q) {
+            if (here) bpe_write_row(len_out, row, n, g, T, [&](int q) {
                 const uint32_t l = __umulhi(2u * (uint32_t)q + 1u, inv);
                 return lds_u16(col0 + 2 * (((uint32_t)q - l * Pp) * STRIDE + l));
             });
@@ -698,9 +728,10 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
         }
         if (WIN) {
             if (g == 0) counts[wi] = round >= max_rounds ? -1 : n;
-        } else if (g == 0) {
+        } else if (g == 0 && here) {
             counts[row] = n;
-            const int32_t bits = bpe_put_length(len_out, row, n) | (round >= max_rounds ? 2 : 0);
+            int32_t bits = bpe_put_length(len_out, row, n) | (round >= max_rounds ? 2 : 0);
+            if (G > 1 && !list && n64 > direct_limit) bits = 8;                               // longer than the hint: left empty
             bpe_put_status(status, row, bits, len_out.store_status != 0 && !list);   // binned rows were written by the binning pass
         }
         team_sync<W, BW, BAR0>(team);
@@ -708,7 +739,7 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
 }
 
 // W: warps per word.  WIN: the words are windows of long rows, their number is *list_count.
-template <int W, bool WIN = false>
+template <int W, bool WIN = false, int G = 1>
 __global__ void __launch_bounds__(bpe_block_warps(W) * 32, bpe_min_blocks(W))
 bpe_lanes_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets,
                  const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
@@ -719,7 +750,7 @@ bpe_lanes_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ 
     extern __shared__ uint4 bpe_dyn[];
     BPE_LANES_SHARED(BW, sh);
     bpe_lanes_setup<BW>(sh, t);
-    bpe_lanes_body<W, BW, 1, (int)bpe_team_bytes(W), false, WIN>(sh, BpeSmemTable{}, reinterpret_cast<uint16_t*>(bpe_dyn), bytes, offsets,
+    bpe_lanes_body<W, BW, 1, (int)bpe_team_bytes(W), false, WIN, G>(sh, BpeSmemTable{}, reinterpret_cast<uint16_t*>(bpe_dyn), bytes, offsets,
                                                                  list, WIN || list ? *list_count : n_direct, work_counter, t, out_tok,
                                                                  counts, status, len_out, direct_limit);
 }
@@ -728,7 +759,7 @@ bpe_lanes_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ 
 // 32 warps per SM, the table copied in once per block, every lookup of the general mode answered from it.
 constexpr int BPE_ST_WARPS = 32;
 __host__ __device__ constexpr size_t bpe_st_team_area(int W) { return (size_t)(BPE_ST_WARPS / W) * bpe_team_bytes(W); }
-template <int W, bool WIN = false>
+template <int W, bool WIN = false, int G = 1>
 __global__ void __launch_bounds__(BPE_ST_WARPS * 32, 1)
 bpe_lanes_st_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets,
                     const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
@@ -751,13 +782,43 @@ bpe_lanes_st_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict
         // block ask for (words are claimed from one counter, and the blocks that start first would otherwise
         // take them all while other SMs stay idle).
         const int n_words = WIN || list ? *list_count : n_direct;
-        const int active = (n_words + (int)gridDim.x - 1) / (int)gridDim.x;
+        const int active = (n_words + (int)gridDim.x * G - 1) / ((int)gridDim.x * G);
         if ((int)(threadIdx.x >> 5) / W >= active) return;
     }
     // sixteen teams of two warps need sixteen hardware barriers: barrier 0 is theirs as well once the set-up is over
-    bpe_lanes_body<W, BPE_ST_WARPS, (W == 2 ? 0 : 1), (int)bpe_team_bytes(W), true, WIN>(sh, stab, reinterpret_cast<uint16_t*>(bpe_dyn),
+    bpe_lanes_body<W, BPE_ST_WARPS, (W == 2 ? 0 : 1), (int)bpe_team_bytes(W), true, WIN, G>(sh, stab, reinterpret_cast<uint16_t*>(bpe_dyn),
                                                                      bytes, offsets, list, WIN || list ? *list_count : n_direct,
                                                                      work_counter, t, out_tok, counts, status, len_out, direct_limit);
+}
+
+// Rows of the first length class only, binned by how many of them fit a warp, in one launch: every warp works through
+// the bins from the longest rows down, so the batch has one tail.  Vocabularies of a few thousand tokens bring their
+// packed table into shared memory (ST), as above.
+template <bool ST>
+__global__ void __launch_bounds__(ST ? BPE_ST_WARPS * 32 : 256, ST ? 1 : BPE_LANES_MIN_BLOCKS)
+bpe_short_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets, const int32_t* __restrict__ class_list,
+                 int64_t n_rows, const int32_t* __restrict__ class_count, int32_t* __restrict__ work, BpeDeviceTable t,
+                 uint16_t* __restrict__ out_tok, int32_t* __restrict__ counts, int32_t* __restrict__ status, BpeLengths len_out) {
+    constexpr int BW = ST ? BPE_ST_WARPS : 8;
+    extern __shared__ uint4 bpe_dyn[];
+    BPE_LANES_SHARED(BW, sh);
+    BpeSmemTable stab{};
+    if (ST) {
+        uint4* const tab = bpe_dyn + bpe_st_team_area(1) / 16;
+        for (uint32_t i = threadIdx.x; i < t.compact_bytes / 16; i += BW * 32) tab[i] = __ldg(t.compact + i);
+        const uint32_t base = smem_u32(tab);
+        stab = BpeSmemTable{base, base + t.compact_slot, base + t.compact_info, t.compact_last};
+    }
+    bpe_lanes_setup<BW>(sh, t);
+    uint16_t* const sm = reinterpret_cast<uint16_t*>(bpe_dyn);
+#define BPE_BIN(K, LIST)                                                                                                      \
+    bpe_lanes_body<1, BW, 1, (int)bpe_team_bytes(1), ST, false, (1 << K)>(sh, stab, sm, bytes, offsets, LIST,                  \
+        class_count[K ? BPE_SHORT_COUNT + K : 0], work + (K ? BPE_SHORT_COUNT + K : 0), t, out_tok, counts, status, len_out, 0);
+    BPE_BIN(0, class_list)
+    BPE_BIN(1, class_list + 2 * n_rows - 1)
+    BPE_BIN(2, class_list + 3 * n_rows - 1)
+    BPE_BIN(3, class_list + 4 * n_rows - 1)
+#undef BPE_BIN
 }
 
 // Rows of several length classes in one launch: a block of BPE_MIXED_WARPS warps works through the classes

@@ -264,7 +264,7 @@ BpeScratch bpe_scratch_layout(const dnatok_handle* h, void* base, int64_t n_rows
 
 // Resident blocks per SM of every merge kernel on a device; filling it also sets the kernels'
 // shared-memory attribute, so a later launch does nothing but launch.
-struct BpeLaunchInfo { int lanes[BPE_LONG_CLASS]; int mixed; int st_room[BPE_LONG_CLASS]; };   // resident blocks per SM of every merge kernel; st_room: bytes a shared-memory table may take beside the teams of each width (0: kernel not usable)
+struct BpeLaunchInfo { int lanes[BPE_LONG_CLASS]; int mixed; int st_room[BPE_LONG_CLASS]; int short_blocks, short_room; };   // resident blocks per SM of every merge kernel; st_room: bytes a shared-memory table may take beside the teams of each width (0: kernel not usable)
 
 constexpr int BPE_WIN_MAX_TEAM = 8;   // widest team that works on a window of a long word (four positions per lane)
 
@@ -281,6 +281,11 @@ int bpe_setup_st(int* room) {
     CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_st_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     if constexpr (W <= BPE_WIN_MAX_TEAM)
         CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_st_kernel<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    if constexpr (W == 1) {
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_st_kernel<1, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_st_kernel<1, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_st_kernel<1, false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    }
     *room = (int)(dyn - (int64_t)bpe_st_team_area(W));
     return 0;
 }
@@ -292,6 +297,11 @@ int bpe_setup_lanes(int* bps) {
     CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if constexpr (W <= BPE_WIN_MAX_TEAM)
         CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_kernel<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if constexpr (W == 1) {
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_kernel<1, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_kernel<1, false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_TRY(cudaFuncSetAttribute(bpe_lanes_kernel<1, false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, bpe_lanes_kernel<W>, BW * 32, smem));
     if (*bps < 1) *bps = 1;
     return 0;
@@ -313,6 +323,20 @@ int bpe_launch_info(int dev, const BpeLaunchInfo** out) {
             (rc = bpe_setup_st<4>(&li.st_room[2])) || (rc = bpe_setup_st<8>(&li.st_room[3])) ||
             (rc = bpe_setup_st<16>(&li.st_room[4])) || (rc = bpe_setup_st<32>(&li.st_room[5])))
             return rc;
+        {
+            cudaFuncAttributes sa;
+            CUDA_TRY(cudaFuncGetAttributes(&sa, bpe_short_kernel<true>));
+            int most = 0;
+            CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+            const int64_t dyn = (int64_t)most - (int64_t)sa.sharedSizeBytes;
+            if (dyn > (int64_t)bpe_st_team_area(1)) {
+                CUDA_TRY(cudaFuncSetAttribute(bpe_short_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+                li.short_room = (int)(dyn - (int64_t)bpe_st_team_area(1));
+            }
+            CUDA_TRY(cudaFuncSetAttribute(bpe_short_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * bpe_team_bytes(1)));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&li.short_blocks, bpe_short_kernel<false>, 256, 8 * bpe_team_bytes(1)));
+            if (li.short_blocks < 1) li.short_blocks = 1;
+        }
         CUDA_TRY(cudaFuncSetAttribute(bpe_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bpe_mixed_bytes()));
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&li.mixed, bpe_mixed_kernel, BPE_MIXED_WARPS * 32, bpe_mixed_bytes()));
         if (li.mixed < 1) li.mixed = 1;
@@ -336,12 +360,13 @@ int bpe_launch_info(int dev, const BpeLaunchInfo** out) {
     return 0;
 }
 
-// Class CLS's rows through teams of W warps (W >= 1 << CLS).
-template <int CLS, int W>
+// Class CLS's rows through teams of W warps (W >= 1 << CLS), or through warps that take G rows at once (direct rows only).
+template <int CLS, int W, int G = 1>
 int launch_bpe_lanes(const DeviceTables& d, const BpeLaunchInfo& li, const BpeDeviceTable& t, const uint8_t* bytes,
                      const int64_t* offsets, int64_t n_rows, const BpeScratch& s, int32_t* status, const BpeLengths& lo,
                      bool direct, cudaStream_t st) {
     constexpr int WI = W == 1 ? 0 : W == 2 ? 1 : W == 4 ? 2 : W == 8 ? 3 : W == 16 ? 4 : 5;
+    constexpr int LIMIT = bpe_class_capacity(CLS) / G;         // longest row
     if (t.compact && g_bpe_smem_table.load() && t.compact_bytes <= (uint32_t)li.st_room[WI]) {
         // the whole merge table fits into shared memory beside the teams: one block of 32 warps per SM
         constexpr int ST_TEAMS = BPE_ST_WARPS / W;
@@ -351,7 +376,7 @@ int launch_bpe_lanes(const DeviceTables& d, const BpeLaunchInfo& li, const BpeDe
         // Rows that are not binned and fit the grid's teams in one go need no work counter: every team takes the word
         // its position names.  Then nothing is zeroed before the launch, the launch before this one in the stream is
         // a kernel as a rule, and programmatic stream serialisation lets this grid's blocks be placed while it drains.
-        const bool one_wave = direct && n_rows <= grid * ST_TEAMS;
+        const bool one_wave = direct && n_rows <= grid * ST_TEAMS * G;
         if (direct && !one_wave) CUDA_TRY(cudaMemsetAsync(s.work + CLS, 0, 4, st));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)grid);
@@ -366,8 +391,8 @@ int launch_bpe_lanes(const DeviceTables& d, const BpeLaunchInfo& li, const BpeDe
         const int32_t* list = direct ? nullptr : s.class_list + (int64_t)CLS * n_rows;
         const int32_t* list_count = s.class_count + CLS;
         int32_t* work = one_wave ? nullptr : s.work + CLS;
-        cudaLaunchKernelEx(&cfg, bpe_lanes_st_kernel<W>, bytes, offsets, list, list_count, work, t, s.tokens, s.counts, status, lo,
-                           (int32_t)n_rows, (int32_t)bpe_class_capacity(CLS));
+        cudaLaunchKernelEx(&cfg, bpe_lanes_st_kernel<W, false, G>, bytes, offsets, list, list_count, work, t, s.tokens, s.counts, status,
+                           lo, (int32_t)n_rows, (int32_t)LIMIT);
         LAUNCH_CHECK("bpe_lanes_st_kernel");
         return 0;
     }
@@ -376,14 +401,14 @@ int launch_bpe_lanes(const DeviceTables& d, const BpeLaunchInfo& li, const BpeDe
     const size_t smem = (size_t)TEAMS * bpe_team_bytes(W);
     // Resident-size grid: every team pulls words from the class's shared counter.
     int64_t grid = (int64_t)d.sm_count * li.lanes[WI];
-    const int64_t need = (n_rows + TEAMS - 1) / TEAMS;
+    const int64_t need = (n_rows + TEAMS * G - 1) / (TEAMS * G);
     if (grid > need) grid = need;
     if (grid < 1) grid = 1;
     const bool one_wave = direct && grid == need;             // as above: no counter to claim from, none to zero
     if (direct && !one_wave) CUDA_TRY(cudaMemsetAsync(s.work + CLS, 0, 4, st));
-    bpe_lanes_kernel<W><<<(unsigned)grid, BW * 32, smem, st>>>(
+    bpe_lanes_kernel<W, false, G><<<(unsigned)grid, BW * 32, smem, st>>>(
         bytes, offsets, direct ? nullptr : s.class_list + (int64_t)CLS * n_rows, s.class_count + CLS,
-        one_wave ? nullptr : s.work + CLS, t, s.tokens, s.counts, status, lo, (int32_t)n_rows, (int32_t)bpe_class_capacity(CLS));
+        one_wave ? nullptr : s.work + CLS, t, s.tokens, s.counts, status, lo, (int32_t)n_rows, (int32_t)LIMIT);
     LAUNCH_CHECK("bpe_lanes_kernel");
     return 0;
 }
@@ -418,6 +443,17 @@ int bpe_team_width(const DeviceTables& d, const BpeLaunchInfo& li, int64_t n_row
     int w = 1;
     while (2 * w <= widest && (int64_t)(2 * w) * n_rows <= slots && (int64_t)(2 * w) * 128 <= max_row) w *= 2;
     return w;
+}
+
+// Rows a warp takes at once when none is longer than max_row.  As few as keep the batch in one wave of resident warps
+// (sharing a warp lengthens a row's rounds, a second wave doubles the time), as many as fit beyond that.  Vocabulary
+// 4,096, rows of 150 bytes, 1 / 2 / 4 per warp: 4,000 rows 18.5 / 18.5 / 21.5 us, 8,000 rows 39.0 / 22.3 / 23.6 us,
+// 16,000 rows 65.5 / 45.2 / 29.2 us; rows of 512 bytes, 1 / 2 per warp: 4,000 rows 25.8 / 31.0 us, 8,000 rows 53.3 / 38.8 us.
+int bpe_rows_per_warp(const DeviceTables& d, const BpeLaunchInfo& li, int64_t n_rows, int64_t max_row) {
+    const int64_t warps = (int64_t)d.sm_count * li.lanes[0] * 8;         // li.lanes[0]: blocks of 8 warps per SM
+    int g = 1;
+    while (g < (1 << BPE_SHORT_BINS) && max_row * 2 * g <= bpe_class_capacity(0) && n_rows > warps * g) g *= 2;
+    return g;
 }
 
 // Where the windows of the long words live: in the long class's working area, which bpe_long_kernel uses for the words
@@ -526,13 +562,21 @@ int run_bpe_merge(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes,
                         id_bits, rf.mask_bits, status_unset ? 1 : 0};
     // One class only, by the caller's bounds on the row lengths: the rows need no binning, the class's kernel
     // takes them as they come (and flags a row the bounds misstated).
-    const bool direct = h->hint_max_row > 0 && (class_mask & (class_mask - 1)) == 0 && !((class_mask >> BPE_LONG_CLASS) & 1u);
+    const bool one_class = h->hint_max_row > 0 && (class_mask & (class_mask - 1)) == 0 && !((class_mask >> BPE_LONG_CLASS) & 1u);
+    // Rows of the first class by the bounds, but shorter on average than their longest: binned by how many fit a warp,
+    // where sharing by the longest row gives two at most.  65,536 rows of 50 to 300 bytes, vocabulary 4,096: one row per
+    // warp 205 us, two (no binning) 154 us, binned 127 us with the binning pass.
+    const int widen = bpe_team_width(d, *li, n_rows, max_row);
+    const bool may_share = h->hint_max_row > 0 && class_mask == 1u && widen == 1;
+    const int share = may_share ? bpe_rows_per_warp(d, *li, n_rows, max_row) : 1;
+    const bool short_bins = may_share && share <= 2 && share < bpe_rows_per_warp(d, *li, n_rows, total_bytes / n_rows);
+    const bool direct = one_class && !short_bins;
     // class_count, work and long_cursor are adjacent; rows that are not binned need at most their class's work counter,
     // which launch_bpe_lanes zeroes when it uses it
     if (!direct) CUDA_TRY(cudaMemsetAsync(s.class_count, 0, 192, st));
     if (!direct) {
         bpe_classify_kernel<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(offsets, n_rows, s.class_count,
-                                                                           s.class_list, s.counts, status, class_mask, lo);
+                                                                           s.class_list, s.counts, status, class_mask, lo, short_bins);
         LAUNCH_CHECK("bpe_classify_kernel");
     }
     BpeDeviceTable t{d.disp, reinterpret_cast<const uint2*>(d.slots), d.merge_out, reinterpret_cast<const uint2*>(d.hot),
@@ -565,7 +609,17 @@ int run_bpe_merge(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes,
         LAUNCH_CHECK("bpe_long_kernel");
     }
     int rc;
-    const int widen = bpe_team_width(d, *li, n_rows, max_row);
+    if (short_bins) {
+        if (t.compact && g_bpe_smem_table.load() && t.compact_bytes <= (uint32_t)li->short_room) {
+            bpe_short_kernel<true><<<(unsigned)d.sm_count, BPE_ST_WARPS * 32, bpe_st_team_area(1) + t.compact_bytes, st>>>(
+                bytes, offsets, s.class_list, n_rows, s.class_count, s.work, t, s.tokens, s.counts, status, lo);
+        } else {
+            bpe_short_kernel<false><<<(unsigned)(d.sm_count * li->short_blocks), 256, 8 * bpe_team_bytes(1), st>>>(
+                bytes, offsets, s.class_list, n_rows, s.class_count, s.work, t, s.tokens, s.counts, status, lo);
+        }
+        LAUNCH_CHECK("bpe_short_kernel");
+        return 0;
+    }
     if (!direct && g_bpe_mixed.load()) {
         // the classes below the widest in one launch, every class at the width of its own or the batch's, whichever is wider
         BpeMixedLevels lv{};
@@ -585,6 +639,9 @@ int run_bpe_merge(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes,
         }
         return 0;
     }
+    if (share == 8) return launch_bpe_lanes<0, 1, 8>(d, *li, t, bytes, offsets, n_rows, s, status, lo, true, st);
+    if (share == 4) return launch_bpe_lanes<0, 1, 4>(d, *li, t, bytes, offsets, n_rows, s, status, lo, true, st);
+    if (share == 2) return launch_bpe_lanes<0, 1, 2>(d, *li, t, bytes, offsets, n_rows, s, status, lo, true, st);
 #define BPE_CLASS(CLS)                                                                                              \
     if (((class_mask >> CLS) & 1u) && (rc = launch_bpe_class<CLS>(d, *li, t, bytes, offsets, n_rows, s, status, lo, direct, widen, st))) \
         return rc;
