@@ -352,6 +352,8 @@ int bpe_launch_info(int dev, const BpeLaunchInfo** out) {
         CUDA_TRY(cudaFuncGetAttributes(&fa, scan_lengths_kernel));
         CUDA_TRY(cudaFuncGetAttributes(&fa, emit_padded_kernel<uint16_t, int64_t, false, EMIT_SPAN>));
         CUDA_TRY(cudaFuncGetAttributes(&fa, emit_padded_kernel<uint16_t, int32_t, false, EMIT_SPAN>));
+        CUDA_TRY(cudaFuncGetAttributes(&fa, emit_short_kernel<uint16_t, int64_t, false>));
+        CUDA_TRY(cudaFuncGetAttributes(&fa, emit_short_kernel<uint16_t, int32_t, false>));
         CUDA_TRY(cudaFuncGetAttributes(&fa, emit_ragged_kernel<uint16_t, int64_t, false>));
         CUDA_TRY(cudaFuncGetAttributes(&fa, emit_ragged_kernel<uint16_t, int32_t, false>));
         it = info.emplace(dev, li).first;
@@ -659,12 +661,21 @@ int launch_emit(const DeviceTables& d, const SrcT* src, const int64_t* offsets, 
         const uint8_t* sb = reinterpret_cast<const uint8_t*>(src);
         const uint8_t* se = sb + (size_t)total_bytes * sizeof(SrcT);
         // 32-bit ids on rows of several thousand columns: wider spans, so a trip stores 4 KiB as it does for 64-bit ids
+        // Flat for short rows (where the line lies: emit_short_kernel) and for small batches, whose time is the kernel's
+        // latency: 200,000 elements take 2.7 us flat and 3.6 us in spans, whatever the rows' length.
+        const int64_t elements = n_rows * rf.out_stride;
+        const bool flat = elements <= (1 << 18) || (elements < (1ll << 30) && rf.out_stride <= (id_bits == 64 ? 128 : 320));
         const bool wide = id_bits == 32 && sizeof(SrcT) == 1 && rf.out_stride >= 4 * EMIT_SPAN_WIDE;
         const int64_t span_cols = wide ? EMIT_SPAN_WIDE : EMIT_SPAN;
         const int64_t spr = (rf.out_stride + span_cols - 1) / span_cols;
         const int64_t n_spans = spr * n_rows;
         const int64_t blocks = (n_spans + EMIT_WARPS - 1) / EMIT_WARPS;
-        const unsigned grid = (unsigned)(blocks < (int64_t)d.sm_count * 32 ? blocks : (int64_t)d.sm_count * 32);
+        unsigned grid = (unsigned)(blocks < (int64_t)d.sm_count * 32 ? blocks : (int64_t)d.sm_count * 32);
+        if (flat) {
+            const int64_t vectors = (elements * (id_bits / 8) + 15) / 16;
+            const int64_t need = (vectors + EMIT_THREADS - 1) / EMIT_THREADS;
+            grid = (unsigned)(need < (int64_t)d.sm_count * 32 ? need : (int64_t)d.sm_count * 32);
+        }
         // programmatic stream serialisation, as for the k-mer row kernel
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(grid);
@@ -676,7 +687,13 @@ int launch_emit(const DeviceTables& d, const SrcT* src, const int64_t* offsets, 
         cfg.attrs = attr;
         cfg.numAttrs = g_emit_overlap_launch.load() ? 1 : 0;
         const int32_t* lut = d.lut256;
-        if (id_bits == 64)
+        if (flat && id_bits == 64)
+            cudaLaunchKernelEx(&cfg, emit_short_kernel<SrcT, int64_t, LUT>, src, offsets, counts, n_rows, lut, rf, (int64_t*)ids, mask,
+                               lengths, status);
+        else if (flat)
+            cudaLaunchKernelEx(&cfg, emit_short_kernel<SrcT, int32_t, LUT>, src, offsets, counts, n_rows, lut, rf, (int32_t*)ids, mask,
+                               lengths, status);
+        else if (id_bits == 64)
             cudaLaunchKernelEx(&cfg, emit_padded_kernel<SrcT, int64_t, LUT, EMIT_SPAN>, src, sb, se, offsets, counts, n_rows, lut, rf,
                                (int64_t*)ids, mask, lengths, status, spr, n_spans);
         else if (wide)
@@ -687,16 +704,17 @@ int launch_emit(const DeviceTables& d, const SrcT* src, const int64_t* offsets, 
                                (int32_t*)ids, mask, lengths, status, spr, n_spans);
         LAUNCH_CHECK("emit_padded_kernel");
     } else {
+        const uint8_t* sb = reinterpret_cast<const uint8_t*>(src);
+        const uint8_t* se = sb + (size_t)total_bytes * sizeof(SrcT);
         const int64_t bound = total_bytes + 2 * n_rows;
-        const int64_t n_tiles = (bound + EMIT_TILE - 1) / EMIT_TILE;
-        if (n_tiles == 0) return 0;
-        const unsigned grid = (unsigned)(n_tiles < (int64_t)d.sm_count * 64 ? n_tiles : (int64_t)d.sm_count * 64);
+        const int64_t blocks = (bound + RAGGED_SPAN * EMIT_WARPS - 1) / (RAGGED_SPAN * EMIT_WARPS);
+        const unsigned grid = (unsigned)(blocks < (int64_t)d.sm_count * 32 ? blocks : (int64_t)d.sm_count * 32);
         if (id_bits == 64)
-            emit_ragged_kernel<SrcT, int64_t, LUT><<<grid, EMIT_THREADS, 0, st>>>(src, offsets, out_offsets, n_rows, d.lut256, rf,
-                                                                                  (int64_t*)ids, mask, n_tiles);
+            emit_ragged_kernel<SrcT, int64_t, LUT><<<grid, EMIT_THREADS, 0, st>>>(src, sb, se, offsets, out_offsets, n_rows, d.lut256, rf,
+                                                                                  (int64_t*)ids, mask);
         else
-            emit_ragged_kernel<SrcT, int32_t, LUT><<<grid, EMIT_THREADS, 0, st>>>(src, offsets, out_offsets, n_rows, d.lut256, rf,
-                                                                                  (int32_t*)ids, mask, n_tiles);
+            emit_ragged_kernel<SrcT, int32_t, LUT><<<grid, EMIT_THREADS, 0, st>>>(src, sb, se, offsets, out_offsets, n_rows, d.lut256, rf,
+                                                                                  (int32_t*)ids, mask);
         LAUNCH_CHECK("emit_ragged_kernel");
     }
     return 0;
