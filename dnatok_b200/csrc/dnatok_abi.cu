@@ -117,6 +117,7 @@ struct dnatok_handle {
     std::vector<int32_t> start_lut;    // char: 256 ids of a row's first character; empty: same as lut256
     std::vector<int32_t> table5, exp_off, exp_ids;   // table-driven k-mer handles (dnatok_create_kmer_table)
     bool kmer_table = false;
+    bool kmer_table_clean = false;     // ... whose clean windows are one token each (kmer_ids) and no window gives none
     int tail_singles = 1;
     int32_t kmer_affine_base = -1;     // >= 0 when kmer_ids[i] == base + i for every i
     bool lut_identity = false;         // char: id == byte value for every byte (byte-level tokenizers)
@@ -162,7 +163,7 @@ int tables_for_current_device(dnatok_handle* h, DeviceTables** out) {
         CUDA_TRY(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
         int rc = upload(&d.lut256, h->lut256);
         if (rc) return rc;
-        if (h->kind == DNATOK_KIND_KMER && !h->kmer_table && (rc = upload(&d.kmer_ids, h->kmer_ids))) return rc;
+        if (h->kind == DNATOK_KIND_KMER && !h->kmer_ids.empty() && (rc = upload(&d.kmer_ids, h->kmer_ids))) return rc;
         if (h->kmer_table) {
             if ((rc = upload(&d.table5, h->table5))) return rc;
             if ((rc = upload(&d.exp_off, h->exp_off))) return rc;
@@ -850,6 +851,44 @@ void launch_kmer_warp(int k, const DeviceTables& d, int32_t affine_base, const u
 #undef KCASE
 }
 
+template <bool TABLE>
+void launch_kmer_count(int k, const uint8_t* bytes, const int64_t* offsets, int64_t n_rows, int64_t total_bytes, const KmerTable& t,
+                       const RowFormat& rf, int32_t* lengths, int32_t* status, cudaStream_t st) {
+    const unsigned grid = (unsigned)((n_rows + KW_WARPS - 1) / KW_WARPS);
+#define KCASE(KK) case KK: kmer_warp_count_kernel<KK, TABLE><<<grid, KW_WARPS * 32, 0, st>>>(bytes, offsets, n_rows, total_bytes, t, rf, \
+                                                                                         lengths, status); break;
+    switch (k) { KCASE(1) KCASE(2) KCASE(3) KCASE(4) KCASE(5) KCASE(6) KCASE(7) KCASE(8) }
+#undef KCASE
+}
+
+template <typename IdT>
+void launch_kmer_table_rows(int k, const DeviceTables& d, const KmerTable& t, const uint8_t* bytes, const int64_t* offsets,
+                            int64_t n_rows, int64_t total_bytes, const RowFormat& rf, void* ids, void* mask, const int32_t* lengths_in,
+                            int32_t* lengths_out, const int64_t* out_offsets, int32_t* status, cudaStream_t st) {
+    // mask and launch attribute as in launch_kmer_warp_k
+    const bool fuse = mask && rf.mask_bits == (int)sizeof(IdT) * 8 &&
+                      ((reinterpret_cast<uintptr_t>(mask) ^ reinterpret_cast<uintptr_t>(ids)) & 15) == 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((n_rows + KW_ROW_WARPS - 1) / KW_ROW_WARPS));
+    cfg.blockDim = dim3(KW_ROW_WARPS * 32);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_kmer_overlap_launch.load() ? 1 : 0;
+    const int32_t* kmer_ids = d.kmer_ids;
+    IdT* ids_t = (IdT*)ids;
+#define KCASE(KK) case KK:                                                                                                             \
+        if (fuse) cudaLaunchKernelEx(&cfg, kmer_warp_table_rows_kernel<IdT, KK, true>, bytes, offsets, n_rows, total_bytes, kmer_ids, t, \
+                                     rf, ids_t, mask, lengths_in, lengths_out, out_offsets, status);                                   \
+        else cudaLaunchKernelEx(&cfg, kmer_warp_table_rows_kernel<IdT, KK, false>, bytes, offsets, n_rows, total_bytes, kmer_ids, t, rf, \
+                                ids_t, mask, lengths_in, lengths_out, out_offsets, status);                                            \
+        break;
+    switch (k) { KCASE(1) KCASE(2) KCASE(3) KCASE(4) KCASE(5) KCASE(6) KCASE(7) KCASE(8) }
+#undef KCASE
+}
+
 // With a scratch buffer, batches of few or very long rows are encoded (and counted) as row segments.
 // Otherwise rows of ordinary length go one per warp and batches of very long rows one per block.
 constexpr int64_t KMER_WARP_MAX_AVG_LEN = 32768;
@@ -872,9 +911,25 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
         need_zero = false;
         return 0;
     };
+    const KmerTable t{d.table5, d.exp_off, d.exp_ids, d.lut256, k, h->tail_singles};
+    if (h->kmer_table_clean) {
+        if (COUNT_ONLY) {
+            if (int rc = zero_now()) return rc;
+            launch_kmer_count<true>(k, bytes, offsets, n_rows, total_bytes, t, rf, lengths_out, status, st);
+            LAUNCH_CHECK("kmer_warp_count_kernel");
+            return 0;
+        }
+        RowFormat rfw = rf;
+        if (need_zero) { rfw.store_status = 1; need_zero = false; }
+        if (id_bits == 64) launch_kmer_table_rows<int64_t>(k, d, t, bytes, offsets, n_rows, total_bytes, rfw, ids, mask, lengths_in,
+                                                           lengths_out, out_offsets, status, st);
+        else launch_kmer_table_rows<int32_t>(k, d, t, bytes, offsets, n_rows, total_bytes, rfw, ids, mask, lengths_in, lengths_out,
+                                             out_offsets, status, st);
+        LAUNCH_CHECK("kmer_warp_table_rows_kernel");
+        return 0;
+    }
     if (h->kmer_table) {
         if (int rc = zero_now()) return rc;
-        const KmerTable t{d.table5, d.exp_off, d.exp_ids, d.lut256, k, h->tail_singles};
         const unsigned grid = (unsigned)((n_rows + KT_WARPS - 1) / KT_WARPS);
         if (id_bits == 64)
             kmer_table_kernel<int64_t, COUNT_ONLY><<<grid, KT_WARPS * 32, 0, st>>>(bytes, offsets, n_rows, t, rf, (int64_t*)ids, mask,
@@ -926,11 +981,7 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
         }
     }
     if (COUNT_ONLY && total_bytes / n_rows <= KMER_WARP_MAX_AVG_LEN) {
-        const unsigned grid = (unsigned)((n_rows + KW_WARPS - 1) / KW_WARPS);
-#define KCASE(KK) case KK: kmer_warp_count_kernel<KK><<<grid, KW_WARPS * 32, 0, st>>>(bytes, offsets, n_rows, total_bytes, rf, \
-                                                                                  lengths_out, status); break;
-        switch (k) { KCASE(1) KCASE(2) KCASE(3) KCASE(4) KCASE(5) KCASE(6) KCASE(7) KCASE(8) }
-#undef KCASE
+        launch_kmer_count<false>(k, bytes, offsets, n_rows, total_bytes, t, rf, lengths_out, status, st);
         LAUNCH_CHECK("kmer_warp_count_kernel");
         return 0;
     }
@@ -1191,6 +1242,19 @@ int dnatok_create_kmer_table(int k, const int32_t* table5, const int32_t* run_of
     if (n_runs) {
         h->exp_off.assign(run_offsets, run_offsets + n_runs + 1);
         h->exp_ids.assign(run_ids, run_ids + run_offsets[n_runs]);
+    }
+    {
+        bool clean = true;
+        for (int32_t e = 0; e < n_runs; ++e) clean = clean && run_offsets[e + 1] > run_offsets[e];
+        h->kmer_ids.resize((size_t)1 << (2 * k));
+        for (size_t i = 0; i < h->kmer_ids.size() && clean; ++i) {
+            size_t i5 = 0;
+            for (int j = k - 1; j >= 0; --j) i5 = i5 * 5 + ((i >> (2 * j)) & 3);
+            clean = table5[i5] >= 0;
+            h->kmer_ids[i] = table5[i5];
+        }
+        h->kmer_table_clean = clean;
+        if (!clean) h->kmer_ids.clear();
     }
     if (h->exp_off.empty()) h->exp_off.assign(1, 0);
     if (h->exp_ids.empty()) h->exp_ids.assign(1, 0);

@@ -215,64 +215,105 @@ template <typename IdT> struct IdPair;
 template <> struct IdPair<int64_t> { using type = longlong2; };
 template <> struct IdPair<int32_t> { using type = int2; };
 
-// Tokens of windows [w_begin, w_end) of one row, counted by one warp with the encoder's window
-// decoding and no stores; counting stops once `stop_at` tokens are reached.  *done tells whether the
-// whole range was looked at.
+// A k-mer tokenizer given window by window (kmer_table_kernel.cuh): what a window with anything but ACGT turns into.
+struct KmerTable {
+    const int32_t* table5;     // [5^k] id >= 0, or -(e + 1): run e of exp_ids
+    const int32_t* exp_off;    // [n_runs + 1]
+    const int32_t* exp_ids;
+    const int32_t* singles;    // [256] id of a character of the tail
+    int k;
+    int tail_singles;          // 0: the len % k tail gives no tokens
+};
+
 template <int K>
-__device__ __forceinline__ int kmer_count_windows(const uint8_t* __restrict__ src, int len, int64_t room_total, int lane,
-                                                  int w_begin, int w_end, int stop_at, bool* done) {
-    constexpr int NW = (2 * K + 3 + 3) / 4;
-    const int n_full = len / K;
-    int total = 0, w0 = w_begin;
-    for (; w0 < w_end && total < stop_at; w0 += 64) {
-        const int wa = w0 + 2 * lane;
-        const int lim = w0 + 64 < w_end ? w0 + 64 : w_end;
-        const int p = wa * K;
-        int cnt = 0;
-        if (wa + 2 <= lim && wa + 2 <= n_full && (int64_t)p + 2 * K + 8 <= room_total) {
-            const uint8_t* g = src + p;
-            const uint32_t sh = (uint32_t)(reinterpret_cast<uintptr_t>(g) & 3u) * 8u;
-            const uint32_t* gw = reinterpret_cast<const uint32_t*>(g - (sh >> 3));
-            uint32_t w[NW];
+__device__ __forceinline__ int kmer_entry5(const KmerTable& t, const uint8_t* __restrict__ window) {
+    int idx = 0;
 #pragma unroll
-            for (int i = 0; i < NW; ++i) w[i] = __ldg(gw + i);
-            uint32_t dA = 0, dB = 0;
-#pragma unroll
-            for (int i = 0; i < NW - 1; ++i) {
-                const uint32_t r = __funnelshift_r(w[i], w[i + 1], sh);
-                uint32_t c, d;
-                acgt_codes4(r, &c, &d);
-                uint32_t mA = 0, mB = 0;
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int pos = 4 * i + b;
-                    if (pos < K) mA |= 0xFFu << (8 * b);
-                    else if (pos < 2 * K) mB |= 0xFFu << (8 * b);
-                }
-                dA |= d & mA;
-                dB |= d & mB;
-            }
-            cnt = (dA == 0 ? 1 : K) + (dB == 0 ? 1 : K);
-        } else {
-            int lenA = 0, lenB = 0;
-            if (wa < lim) { const int h = len - p; lenA = h < K ? h : K; }
-            if (wa + 1 < lim) { const int h = len - p - K; lenB = h < K ? h : K; }
-            bool okA = lenA == K, okB = lenB == K;
-            for (int i = 0; i < lenA; ++i) okA &= kmer_code(__ldg(src + p + i)) < 4;
-            for (int i = 0; i < lenB; ++i) okB &= kmer_code(__ldg(src + p + K + i)) < 4;
-            cnt = (lenA == 0 ? 0 : (okA ? 1 : lenA)) + (lenB == 0 ? 0 : (okB ? 1 : lenB));
-        }
-        total += __reduce_add_sync(0xffffffffu, cnt);
-    }
-    *done = w0 >= w_end;
-    return total;
+    for (int i = 0; i < K; ++i) idx = idx * 5 + kmer_code(__ldg(window + i));
+    return __ldg(t.table5 + idx);
+}
+__device__ __forceinline__ int kmer_entry_tokens(const KmerTable& t, int entry) {
+    return entry >= 0 ? 1 : __ldg(t.exp_off - entry) - __ldg(t.exp_off - entry - 1);
 }
 
-// Token counts only (the sizing pass for 'longest' padding and for ragged output): one warp per row.
-template <int K>
+// Tokens of windows [w_begin, w_end) of one row, counted by one warp: one per complete window, the letters of a short
+// last window, and what windows with anything but ACGT give beyond one.  The bytes are taken as aligned 16-byte chunks
+// (four per lane in flight), each turned into a mask of the bytes that are not ACGT; a lane looks at the windows that end in
+// its chunk, with the mask of the lane before for where they begin.
+// TABLE: such a window's tokens are those of its table entry, not its K letters.
+// buf_lo, buf_hi: the input buffer; nothing outside it is read.
+template <int K, bool TABLE>
+__device__ __forceinline__ int kmer_count_range(const uint8_t* __restrict__ src, int len, const uint8_t* buf_lo, const uint8_t* buf_hi,
+                                                int lane, int w_begin, int w_end, const KmerTable& t) {
+    constexpr int UNROLL = 4;
+    const int n_full = len / K;
+    const int nf = w_end < n_full ? w_end : n_full;
+    int count = nf > w_begin ? nf - w_begin : 0;
+    if (w_end > n_full) count += len - n_full * K;             // the short window's letters
+    const uint8_t* const g = src + (int64_t)w_begin * K;
+    const int bytes = nf > w_begin ? (nf - w_begin) * K : 0;
+    const int a = (int)(reinterpret_cast<uintptr_t>(g) & 15);
+    const uint8_t* const base = g - a;
+    const int n_chunks = bytes ? (int)(((uint32_t)a + (uint32_t)bytes + 15u) >> 4) : 0;
+    int extra = 0;
+    uint32_t carry = 0;                                        // mask of the chunk before lane 0's
+    for (int c0 = 0; c0 < n_chunks; c0 += 32 * UNROLL) {
+        uint4 v[UNROLL];
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            const int c = c0 + 32 * u + lane;
+            v[u] = make_uint4(0x41414141u, 0x41414141u, 0x41414141u, 0x41414141u);
+            if (c < n_chunks) {
+                const uint8_t* p = base + 16 * (int64_t)c;
+                if (p >= buf_lo && p + 16 <= buf_hi) v[u] = __ldg(reinterpret_cast<const uint4*>(p));
+                else {
+                    uint8_t tmp[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) tmp[i] = (p + i >= buf_lo && p + i < buf_hi) ? __ldg(p + i) : (uint8_t)'A';
+                    v[u] = *reinterpret_cast<uint4*>(tmp);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            const int c = c0 + 32 * u + lane;
+            uint32_t code, d[4];
+            acgt_codes4(v[u].x, &code, &d[0]);
+            acgt_codes4(v[u].y, &code, &d[1]);
+            acgt_codes4(v[u].z, &code, &d[2]);
+            acgt_codes4(v[u].w, &code, &d[3]);
+            if (carry == 0u && !__any_sync(0xffffffffu, (d[0] | d[1] | d[2] | d[3]) != 0u)) continue;
+            uint32_t bad = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {                      // one bit per byte that is not zero
+                const uint32_t m = (((d[i] & 0x7f7f7f7fu) + 0x7f7f7f7fu) | d[i]) & 0x80808080u;
+                bad |= (((m >> 7) * 0x01020408u) >> 24) << (4 * i);
+            }
+            const int from = (int)(16u * (uint32_t)c - (uint32_t)a);   // place of the chunk's first byte among the windows' bytes
+            if (c == 0) bad &= 0xFFFFu << a;
+            if (c >= n_chunks - 1) bad &= c >= n_chunks ? 0u : (0xFFFFu >> (16 - (bytes - from)));   // the last chunk ends with them
+            uint32_t before = __shfl_up_sync(0xffffffffu, bad, 1);
+            if (lane == 0) before = carry;
+            carry = __shfl_sync(0xffffffffu, bad, 31);
+            const uint32_t both = (bad << 16) | before;
+            if (c < n_chunks) {
+                int end = (from < 0 ? K : (from / K + 1) * K) - from;       // behind the first window that ends in the chunk
+#pragma unroll
+                for (int i = 0; i < (15 + K) / K; ++i, end += K)
+                    if (end <= 16 && (both >> (16 + end - K)) & ((1u << K) - 1u))
+                        extra += TABLE ? kmer_entry_tokens(t, kmer_entry5<K>(t, g + (from + end - K))) - 1 : K - 1;
+            }
+        }
+    }
+    return count + __reduce_add_sync(0xffffffffu, extra);
+}
+
+// Token counts only (the sizing pass for 'longest' padding and for ragged output): one warp per row.  Of a row that is
+// cut at cap tokens the first cap + 1 windows decide everything.
+template <int K, bool TABLE>
 __global__ void __launch_bounds__(KW_WARPS * 32)
 kmer_warp_count_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets, int64_t n_rows,
-                       int64_t total_bytes, RowFormat f, int32_t* __restrict__ lengths_out,
+                       int64_t total_bytes, KmerTable t, RowFormat f, int32_t* __restrict__ lengths_out,
                        int32_t* __restrict__ status) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * KW_WARPS + (threadIdx.x >> 5);
@@ -281,14 +322,14 @@ kmer_warp_count_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restr
     const int64_t off = offsets[row];
     const int64_t len64 = offsets[row + 1] - off;
     const int len = (int)(len64 < 0x7fffffff ? len64 : 0x7fffffff);
-    const int n_win = (len + K - 1) / K;
+    const int n_win = len / K + (len % K && (!TABLE || t.tail_singles) ? 1 : 0);
     const int cap = (int)(f.cap_content < 0x7fffffff ? f.cap_content : 0x7fffffff);
-    bool done;
-    const int base = kmer_count_windows<K>(bytes + off, len, total_bytes - off, lane, 0, n_win, cap, &done);
+    const int w_end = n_win <= cap ? n_win : cap + 1;
+    const int base = kmer_count_range<K, TABLE>(bytes + off, len, bytes, bytes + total_bytes, lane, 0, w_end, t);
     if (lane == 0) {
         const int n = base < cap ? base : cap;
         lengths_out[row] = n + n_special;
-        if (status && f.clip_is_error && (base > cap || !done)) atomicOr(status + row, 4);
+        if (status && f.clip_is_error && base > cap) atomicOr(status + row, 4);
     }
 }
 
@@ -312,8 +353,7 @@ kmer_seg_count_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restri
         const int64_t w0 = (int64_t)seg * seg_windows;
         if (w0 >= n_win) continue;
         const int w_end = (seg == n_seg - 1 || w0 + seg_windows >= n_win) ? n_win : (int)w0 + seg_windows;
-        bool done;
-        const int cnt = kmer_count_windows<K>(bytes + off, len, total_bytes - off, lane, (int)w0, w_end, 0x7fffffff, &done);
+        const int cnt = kmer_count_range<K, false>(bytes + off, len, bytes, bytes + total_bytes, lane, (int)w0, w_end, KmerTable{});
         if (lane == 0 && cnt) atomicAdd(counts + row, cnt);
     }
 }
@@ -358,10 +398,12 @@ __device__ __forceinline__ KmerRow<IdT> kmer_row_setup(const uint8_t* bytes, int
 // returns the token count after them (it stops early once the cap is reached) and reports clipping.
 // AFFINE: the 4**K table is base + index (checked on the host), so no gather is needed.
 // FUSE_MASK: the mask has the ids' element type and is stored next to each id (mdelta elements away).
-template <typename IdT, int K, bool AFFINE, bool FUSE_MASK>
+// TABLE: a complete window with anything but ACGT gives the tokens of its entry in table t, not its letters.
+template <typename IdT, int K, bool AFFINE, bool FUSE_MASK, bool TABLE = false>
 __device__ __forceinline__ int kmer_encode_windows(const KmerRow<IdT>& r, int cap, const int32_t* __restrict__ kmer_ids,
                                                    int32_t affine_base, const int32_t* __restrict__ single_ids,
-                                                   int64_t mdelta, int lane, int w, int w_end, int base, bool* clipped) {
+                                                   int64_t mdelta, int lane, int w, int w_end, int base, bool* clipped,
+                                                   const KmerTable& t5 = KmerTable{}) {
     constexpr int NW = (2 * K + 3 + 3) / 4;            // aligned words covering 2K bytes at any byte offset
     constexpr uint32_t IDX_MASK = (1u << (2 * K)) - 1u;
     using Pair = typename IdPair<IdT>::type;
@@ -443,8 +485,16 @@ __device__ __forceinline__ int kmer_encode_windows(const KmerRow<IdT>& r, int ca
             const int left = w_end - w0;
             base += left < nwin ? left : nwin;
         } else {
-            const int cntA = t.lenA == 0 ? 0 : (t.cleanA ? 1 : t.lenA);
-            const int cntB = t.lenB == 0 ? 0 : (t.cleanB ? 1 : t.lenB);
+            int cntA = t.lenA == 0 ? 0 : (t.cleanA ? 1 : t.lenA);
+            int cntB = t.lenB == 0 ? 0 : (t.cleanB ? 1 : t.lenB);
+            int entA = 0, entB = 0;
+            if (TABLE && t.lenA == K && !t.cleanA) { entA = kmer_entry5<K>(t5, src + t.p); cntA = kmer_entry_tokens(t5, entA); }
+            if (TABLE && t.lenB == K && !t.cleanB) { entB = kmer_entry5<K>(t5, src + t.p + K); cntB = kmer_entry_tokens(t5, entB); }
+            auto put_entry = [&](int entry, int cnt, int at) {
+                const int32_t* run = entry < 0 ? t5.exp_ids + __ldg(t5.exp_off - entry - 1) : nullptr;
+                for (int i = 0; i < cnt; ++i, ++at)
+                    if (at < cap) { dst[at] = (IdT)(run ? __ldg(run + i) : entry); if (FUSE_MASK) mdst[at] = 1; }
+            };
             int my = cntA + cntB, x = my;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -455,10 +505,12 @@ __device__ __forceinline__ int kmer_encode_windows(const KmerRow<IdT>& r, int ca
             int pos = base + x - my;
             if (t.lenA) {
                 if (t.cleanA) { if (pos < cap) { dst[pos] = (IdT)__ldg(kmer_ids + t.idxA); if (FUSE_MASK) mdst[pos] = 1; } ++pos; }
+                else if (TABLE && t.lenA == K) { put_entry(entA, cntA, pos); pos += cntA; }
                 else for (int i = 0; i < t.lenA; ++i, ++pos) if (pos < cap) { dst[pos] = (IdT)__ldg(single_ids + __ldg(src + t.p + i)); if (FUSE_MASK) mdst[pos] = 1; }
             }
             if (t.lenB) {
                 if (t.cleanB) { if (pos < cap) { dst[pos] = (IdT)__ldg(kmer_ids + t.idxB); if (FUSE_MASK) mdst[pos] = 1; } ++pos; }
+                else if (TABLE && t.lenB == K) put_entry(entB, cntB, pos);
                 else for (int i = 0; i < t.lenB; ++i, ++pos) if (pos < cap) { dst[pos] = (IdT)__ldg(single_ids + __ldg(src + t.p + K + i)); if (FUSE_MASK) mdst[pos] = 1; }
             }
             base += total;
@@ -654,6 +706,32 @@ kmer_warp_rows_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restri
     bool clipped = false;
     const int base = kmer_encode_windows<IdT, K, AFFINE, FUSE_MASK>(r, cap, kmer_ids, affine_base, single_ids, mdelta, lane,
                                                                     0, r.n_win, 0, &clipped);
+    kmer_finish_row<IdT, FUSE_MASK>(r, row, base, cap, clipped, f, ids, mask, lengths_out, out_offsets, status, lane, long_bit);
+}
+
+// The same for a tokenizer given window by window whose clean windows are one token each (kmer_ids: their ids in 4^K
+// order): clean stretches take the row encoder's loop, the other windows' tokens come from the table.  kmer_table_kernel,
+// which looks every window up from its bytes one by one, took 70 us (and 41 us to size the rows) for 8,190 rows of 500 to
+// 4,000 bp at K = 5, 64-bit ids and mask; here they take 45 us, and 17 us.
+template <typename IdT, int K, bool FUSE_MASK>
+__global__ void __launch_bounds__(KW_ROW_WARPS * 32, KW_BLOCKS_PER_SM)
+kmer_warp_table_rows_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets, int64_t n_rows,
+                            int64_t total_bytes, const int32_t* __restrict__ kmer_ids, KmerTable t, RowFormat f, IdT* __restrict__ ids,
+                            void* __restrict__ mask, const int32_t* __restrict__ lengths_in, int32_t* __restrict__ lengths_out,
+                            const int64_t* __restrict__ out_offsets, int32_t* __restrict__ status) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * KW_ROW_WARPS + (threadIdx.x >> 5);
+    if (row >= n_rows) return;
+    KmerRow<IdT> r = kmer_row_setup<IdT, K>(bytes, offsets[row], offsets[row + 1], row, total_bytes, f, ids, lengths_in, out_offsets);
+    if (!t.tail_singles) r.n_win = r.len / K;
+    const int cap = (int)(f.cap_content < 0x7fffffff ? f.cap_content : 0x7fffffff);
+    const int64_t mdelta = FUSE_MASK ? (reinterpret_cast<IdT*>(mask) - ids) : 0;
+    const int32_t long_bit = offsets[row + 1] - offsets[row] > 0x7fffffff ? 1 : 0;    // cut at 2^31 - 1 bytes and reported
+    bool clipped = false;
+    const int base = kmer_encode_windows<IdT, K, false, FUSE_MASK, true>(r, cap, kmer_ids, 0, t.singles, mdelta, lane, 0, r.n_win, 0,
+                                                                         &clipped, t);
     kmer_finish_row<IdT, FUSE_MASK>(r, row, base, cap, clipped, f, ids, mask, lengths_out, out_offsets, status, lane, long_bit);
 }
 

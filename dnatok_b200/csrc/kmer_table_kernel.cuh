@@ -5,22 +5,13 @@
 // character outside ACGT counts as N, the reference's replace_with_n policy (:1318-1332).  The
 // len % k tail gives one id per character, or nothing for tokenizers that drop it.
 //
-// One warp per row, 32 windows per trip: every lane looks its window up, a warp scan places the
-// runs, the ids are stored.  Rows of such tokenizers are rare and short-listed at discovery, so
-// this kernel is written for clarity; the 4^k kernels in kmer_kernel.cuh carry the bandwidth.
+// Tables whose clean windows are one token each, with no window without a token, run in the 4^k kernels
+// (kmer_warp_table_rows_kernel, kmer_warp_count_kernel); this kernel takes the rest: one warp per row, 32 windows per
+// trip, every lane looks its window up, a warp scan places the runs, the ids are stored.
 #pragma once
 #include "kmer_kernel.cuh"
 
 namespace dnatok {
-
-struct KmerTable {
-    const int32_t* table5;     // [5^k] id >= 0, or -(e + 1): run e of exp_ids
-    const int32_t* exp_off;    // [n_runs + 1]
-    const int32_t* exp_ids;
-    const int32_t* singles;    // [256] id of a character of the tail
-    int k;
-    int tail_singles;          // 0: the len % k tail gives no tokens
-};
 
 constexpr int KT_WARPS = 8;
 

@@ -151,3 +151,66 @@ def test_start_table_tokenizer_on_gpu():
     enc = tok(strs, padding="max_length", max_length=33, truncation=True, add_special_tokens=False, return_tensors="np")
     for i, w in enumerate(want):
         assert enc["input_ids"][i].tolist() == w[:33] + [0] * max(0, 33 - len(w))
+
+
+def _windows_spec(k, seed, runs):
+    """A synthetic tokenizer given window by window: clean windows one id each, the others `runs` ids at most (no more than
+    k: a row never has more tokens than bytes)."""
+    import itertools
+    from dnatok_b200.tables import Specials, TokenizerSpec
+    rng = np.random.default_rng(seed)
+    lut = np.full(256, 1, np.int32)
+    for i, c in enumerate("ACGTN"):
+        lut[ord(c)] = 5 + i
+    table, offsets, ids = [], [0], []
+    for win in itertools.product("ACGTN", repeat=k):
+        if "N" not in win or runs == 1:
+            table.append(int(rng.integers(10, 5000)))
+        else:
+            table.append(-len(offsets))
+            ids += rng.integers(5000, 9000, size=int(rng.integers(1, runs + 1))).tolist()
+            offsets.append(len(ids))
+    return TokenizerSpec("kmer", Specials(0, 1, 2, 3), 9000, lut, k=k, kmer_table5=np.array(table, np.int32),
+                         kmer_run_offsets=np.array(offsets, np.int32), kmer_run_ids=np.array(ids, np.int32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k,runs", [(1, 1), (2, 1), (2, 2), (3, 3), (4, 2), (5, 5), (6, 6), (7, 2), (8, 8)])
+@pytest.mark.parametrize("tail", [True, False])
+def test_clean_window_tables_in_the_row_encoder(k, runs, tail):
+    """Rows around the chunks of 64 and 256 windows and the 16-byte chunks of the sizing pass, an odd start of the buffer,
+    windows with Ns at every place, truncation inside a run."""
+    from dnatok_b200.tokenizer import B200Tokenizer
+    spec = _windows_spec(k, 3 * k + runs, runs)
+    spec.kmer_tail_singles = tail
+    tok = B200Tokenizer(spec)
+    rng = np.random.default_rng(k)
+    lens = [0, 1, k - 1, k, k + 1, 15, 16, 17, 63 * k, 64 * k, 64 * k + 1, 65 * k - 1, 256 * k, 257 * k + 1, 512 * k, 2049 * k + k - 1]
+    lens += rng.integers(0, 700 * k, size=40).tolist()
+    strs = []
+    for i, n in enumerate(lens):
+        x = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, size=n)].copy()
+        x[rng.random(n) < (0.0, 0.002, 0.2)[i % 3]] = ord("N")
+        if n > 40 and i % 4 == 0:
+            x[n // 3:n // 3 + 30] = ord("x")
+        strs.append(x.tobytes().decode())
+    want = [tables.expected_kmer_table_ids(s, spec) for s in strs]
+    data = "".join(strs).encode()
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    d_b = torch.zeros(len(data) + 3, dtype=torch.uint8, device="cuda")[3:]
+    d_b.copy_(torch.from_numpy(np.frombuffer(data, np.uint8).copy()))
+    d_o = torch.from_numpy(offs).cuda()
+    enc = tok.encode_device(d_b, d_o, host_offsets=offs, padding=False, add_special_tokens=False, ids_dtype=torch.int32)
+    ids, oo = enc["input_ids"].cpu().numpy(), enc["offsets"].cpu().numpy()
+    for i, w in enumerate(want):
+        assert ids[oo[i]:oo[i + 1]].tolist() == w, "row %d (%d bytes)" % (i, lens[i])
+    for side in ("right", "left"):
+        tok.padding_side = side
+        for kw, cut in ((dict(padding="longest"), None), (dict(padding="max_length", max_length=131, truncation=True), 129)):
+            enc = tok.encode_device(d_b, d_o, host_offsets=offs, add_special_tokens=True, **kw)
+            got, mask = enc["input_ids"].cpu().numpy(), enc["attention_mask"].cpu().numpy()
+            for i, w in enumerate(want):
+                row = [2] + w[:cut] + [3]
+                pad = [0] * (got.shape[1] - len(row))
+                assert got[i].tolist() == (pad + row if side == "left" else row + pad), (side, kw, i)
+                assert mask[i].sum() == len(row) and enc["lengths"][i].item() == len(row)
