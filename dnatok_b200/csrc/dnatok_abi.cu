@@ -900,7 +900,10 @@ template <bool COUNT_ONLY>
 int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, const int64_t* offsets,
                 int64_t n_rows, int64_t total_bytes, const RowFormat& rf, int id_bits, void* ids, void* mask,
                 const int32_t* lengths_in, int32_t* lengths_out, const int64_t* out_offsets,
-                int32_t* status, void* scratch, size_t scratch_bytes, cudaStream_t st, bool status_unset = false) {
+                int32_t* status, void* scratch, size_t scratch_bytes, cudaStream_t st, bool status_unset = false,
+                bool* segments_counted = nullptr) {
+    // segments_counted: set by the sizing pass when the scratch holds every segment's place in its row, read by an encode
+    // that follows in the same call
     if (n_rows == 0) return 0;
     const int k = h->k;
     // status_unset: the caller left the status words as they were.  The row-per-warp encoder writes every row's word
@@ -952,10 +955,12 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
     // a row that gave up is reported through the status array only: without one the segment encoder is not used
     if (!COUNT_ONLY && status && scratch && !(reinterpret_cast<uintptr_t>(scratch) & 255) && longest < (1ll << 30) &&
         (few_rows || long_rows || g_kmer_force_segments)) {
-        const KmerScratch ks = kmer_scratch_layout(h, scratch, n_rows, total_bytes);
+        KmerScratch ks = kmer_scratch_layout(h, scratch, n_rows, total_bytes);
         if (ks.bytes <= scratch_bytes && (ks.n_seg > 1 || g_kmer_force_segments)) {
             if (int rc = zero_now()) return rc;
-            CUDA_TRY(cudaMemsetAsync(scratch, 0, ks.bytes, st));
+            const bool counted = segments_counted && *segments_counted && g_kmer_test_withhold.load() < 0;
+            if (counted) ks.tickets = nullptr;
+            else CUDA_TRY(cudaMemsetAsync(scratch, 0, ks.bytes, st));
             if (id_bits == 64) launch_kmer_seg<int64_t>(k, d, h->kmer_affine_base, bytes, offsets, n_rows, total_bytes, rf, ids, mask,
                                                         lengths_in, lengths_out, out_offsets, status, ks, st);
             else launch_kmer_seg<int32_t>(k, d, h->kmer_affine_base, bytes, offsets, n_rows, total_bytes, rf, ids, mask,
@@ -968,16 +973,18 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
     if (COUNT_ONLY && scratch && !(reinterpret_cast<uintptr_t>(scratch) & 255) && (few_rows || long_rows)) {
         const KmerScratch ks = kmer_scratch_layout(h, scratch, n_rows, total_bytes);
         if (ks.bytes <= scratch_bytes && ks.n_seg > 1) {
-            int32_t* counts = reinterpret_cast<int32_t*>(ks.flags);
-            CUDA_TRY(cudaMemsetAsync(counts, 0, (size_t)n_rows * 4, st));
             const int64_t want = (n_rows * ks.n_seg + KW_WARPS - 1) / KW_WARPS, most = (int64_t)d.sm_count * 8;
             const unsigned grid = (unsigned)(want < most ? want : most);
 #define KCASE(KK) case KK: kmer_seg_count_kernel<KK><<<grid, KW_WARPS * 32, 0, st>>>(bytes, offsets, n_rows, total_bytes, ks.n_seg, \
-                                                                                 KSEG_WINDOWS, counts); break;
+                                                                                 KSEG_WINDOWS, ks.flags); break;
             switch (k) { KCASE(1) KCASE(2) KCASE(3) KCASE(4) KCASE(5) KCASE(6) KCASE(7) KCASE(8) }
 #undef KCASE
             LAUNCH_CHECK("kmer_seg_count_kernel");
-            return launch_span_lengths(offsets, counts, n_rows, rf, lengths_out, status, st);
+            kmer_seg_total_kernel<<<(unsigned)(n_rows < 65536 ? n_rows : 65536), 256, 0, st>>>(ks.flags, n_rows, ks.n_seg, rf, lengths_out,
+                                                                                           status);
+            LAUNCH_CHECK("kmer_seg_total_kernel");
+            if (segments_counted) *segments_counted = true;
+            return 0;
         }
     }
     if (COUNT_ONLY && total_bytes / n_rows <= KMER_WARP_MAX_AVG_LEN) {
@@ -1341,9 +1348,10 @@ int dnatok_scan_lengths(const int32_t* d_lengths, int64_t n_rows, int64_t* d_out
     return DNATOK_OK;
 }
 
-int dnatok_prepare(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
-                   int64_t total_bytes, const dnatok_format* fmt, int32_t* d_lengths, int32_t* d_status,
-                   void* d_scratch, size_t scratch_bytes, dnatok_stream stream) {
+// segments_counted: see launch_kmer; only dnatok_encode, which owns the scratch between the two steps, passes it.
+static int prepare_rows(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
+                        int64_t total_bytes, const dnatok_format* fmt, int32_t* d_lengths, int32_t* d_status,
+                        void* d_scratch, size_t scratch_bytes, dnatok_stream stream, bool* segments_counted) {
     if (int rc = check_batch(h, d_bytes, d_offsets, n_rows, total_bytes)) return rc;
     if (int rc = check_format(fmt, false)) return rc;
     if (!d_lengths) return fail(DNATOK_ERR_INVALID, "d_lengths is NULL");
@@ -1358,17 +1366,23 @@ int dnatok_prepare(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_of
             return launch_span_lengths(d_offsets, nullptr, n_rows, rf, d_lengths, d_status, st);
         case DNATOK_KIND_KMER:
             return launch_kmer<true>(h, *d, d_bytes, d_offsets, n_rows, total_bytes, rf, 64, nullptr, nullptr, nullptr, d_lengths,
-                                     nullptr, d_status, d_scratch, scratch_bytes, st);
+                                     nullptr, d_status, d_scratch, scratch_bytes, st, false, segments_counted);
         default: {
             return run_bpe_merge(h, *d, d_bytes, d_offsets, n_rows, total_bytes, d_status, d_scratch, scratch_bytes, rf, d_lengths, st);
         }
     }
 }
 
-int dnatok_write(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
-                 int64_t total_bytes, const dnatok_format* fmt, const int32_t* d_lengths,
-                 const int64_t* d_out_offsets, void* d_ids, void* d_mask, int32_t* d_status, void* d_scratch,
-                 size_t scratch_bytes, dnatok_stream stream) {
+int dnatok_prepare(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
+                   int64_t total_bytes, const dnatok_format* fmt, int32_t* d_lengths, int32_t* d_status,
+                   void* d_scratch, size_t scratch_bytes, dnatok_stream stream) {
+    return prepare_rows(h, d_bytes, d_offsets, n_rows, total_bytes, fmt, d_lengths, d_status, d_scratch, scratch_bytes, stream, nullptr);
+}
+
+static int write_rows(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
+                      int64_t total_bytes, const dnatok_format* fmt, const int32_t* d_lengths,
+                      const int64_t* d_out_offsets, void* d_ids, void* d_mask, int32_t* d_status, void* d_scratch,
+                      size_t scratch_bytes, dnatok_stream stream, bool* segments_counted) {
     if (int rc = check_batch(h, d_bytes, d_offsets, n_rows, total_bytes)) return rc;
     if (int rc = check_format(fmt, false)) return rc;
     if (!d_ids && n_rows) return fail(DNATOK_ERR_INVALID, "d_ids is NULL");
@@ -1387,7 +1401,7 @@ int dnatok_write(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offs
             if (fmt->out_stride > 0 && fmt->pad_left && !d_lengths)
                 return fail(DNATOK_ERR_INVALID, "left padding needs d_lengths from dnatok_prepare");
             return launch_kmer<false>(h, *d, d_bytes, d_offsets, n_rows, total_bytes, rf, fmt->id_bits, d_ids, d_mask, d_lengths,
-                                      nullptr, d_out_offsets, d_status, d_scratch, scratch_bytes, st);
+                                      nullptr, d_out_offsets, d_status, d_scratch, scratch_bytes, st, false, segments_counted);
         default: {
             if (!d_scratch) return fail(DNATOK_ERR_SCRATCH, "BPE write needs the scratch filled by dnatok_prepare");
             BpeScratch s = bpe_scratch_layout(h, d_scratch, n_rows, total_bytes);
@@ -1396,6 +1410,14 @@ int dnatok_write(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offs
                                                 d_ids, d_mask, nullptr, d_out_offsets, d_status, st);
         }
     }
+}
+
+int dnatok_write(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
+                 int64_t total_bytes, const dnatok_format* fmt, const int32_t* d_lengths,
+                 const int64_t* d_out_offsets, void* d_ids, void* d_mask, int32_t* d_status, void* d_scratch,
+                 size_t scratch_bytes, dnatok_stream stream) {
+    return write_rows(h, d_bytes, d_offsets, n_rows, total_bytes, fmt, d_lengths, d_out_offsets, d_ids, d_mask, d_status, d_scratch,
+                      scratch_bytes, stream, nullptr);
 }
 
 int dnatok_encode(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
@@ -1425,14 +1447,15 @@ int dnatok_encode(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_off
                               (h->kind == DNATOK_KIND_KMER && fmt->pad_left);
     if (need_prepare) {
         if (!d_lengths) return fail(DNATOK_ERR_INVALID, "this format needs d_lengths");
-        if (int rc = dnatok_prepare(h, d_bytes, d_offsets, n_rows, total_bytes, fmt, d_lengths, d_status, d_scratch,
-                                    scratch_bytes, stream))
+        bool segments_counted = false;
+        if (int rc = prepare_rows(h, d_bytes, d_offsets, n_rows, total_bytes, fmt, d_lengths, d_status, d_scratch,
+                                  scratch_bytes, stream, &segments_counted))
             return rc;
         if (ragged) {
             if (int rc = dnatok_scan_lengths(d_lengths, n_rows, d_out_offsets, stream)) return rc;
         }
-        return dnatok_write(h, d_bytes, d_offsets, n_rows, total_bytes, fmt, d_lengths, d_out_offsets, d_ids, d_mask,
-                            d_status, d_scratch, scratch_bytes, stream);
+        return write_rows(h, d_bytes, d_offsets, n_rows, total_bytes, fmt, d_lengths, d_out_offsets, d_ids, d_mask,
+                          d_status, d_scratch, scratch_bytes, stream, &segments_counted);
     }
     // padded char / right-padded k-mer: one kernel, lengths written on the way
     if (!d_ids && n_rows) return fail(DNATOK_ERR_INVALID, "d_ids is NULL");

@@ -335,11 +335,11 @@ kmer_warp_count_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restr
 
 // The same count for batches of few or very long rows: every warp counts segments of KSEG_WINDOWS
 // windows (ticket t = segment t / n_rows of row t % n_rows, the last segment index without upper
-// bound) and adds them to counts[row], which the caller zeroed and turns into lengths afterwards.
+// bound) into counts[t]; kmer_seg_total_kernel turns them into row lengths.
 template <int K>
 __global__ void __launch_bounds__(KW_WARPS * 32)
 kmer_seg_count_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets, int64_t n_rows,
-                      int64_t total_bytes, int n_seg, int seg_windows, int32_t* __restrict__ counts) {
+                      int64_t total_bytes, int n_seg, int seg_windows, uint32_t* __restrict__ counts) {
     const int lane = threadIdx.x & 31;
     const int64_t n_tickets = n_rows * (int64_t)n_seg;
     const int64_t n_warps = (int64_t)gridDim.x * KW_WARPS;
@@ -351,10 +351,12 @@ kmer_seg_count_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restri
         const int len = (int)(len64 < 0x7fffffff ? len64 : 0x7fffffff);
         const int n_win = (len + K - 1) / K;
         const int64_t w0 = (int64_t)seg * seg_windows;
-        if (w0 >= n_win) continue;
-        const int w_end = (seg == n_seg - 1 || w0 + seg_windows >= n_win) ? n_win : (int)w0 + seg_windows;
-        const int cnt = kmer_count_range<K, false>(bytes + off, len, bytes, bytes + total_bytes, lane, (int)w0, w_end, KmerTable{});
-        if (lane == 0 && cnt) atomicAdd(counts + row, cnt);
+        int cnt = 0;
+        if (w0 < n_win) {
+            const int w_end = (seg == n_seg - 1 || w0 + seg_windows >= n_win) ? n_win : (int)w0 + seg_windows;
+            cnt = kmer_count_range<K, false>(bytes + off, len, bytes, bytes + total_bytes, lane, (int)w0, w_end, KmerTable{});
+        }
+        if (lane == 0) counts[t] = (uint32_t)cnt;
     }
 }
 
@@ -759,6 +761,42 @@ constexpr int KSEG_BLOCKS_PER_SM = 4;    // 64 registers per thread: the decoded
 constexpr int KSEG_POLL_LIMIT = 1 << 20;    // default bound on the polls of one wait
 constexpr uint32_t KSEG_OWN = 1u << 30, KSEG_TOTAL = 2u << 30, KSEG_POISON = 3u << 30, KSEG_VALUE = (1u << 30) - 1u;
 
+// One block per row: the row's length from its segments' counts.  The counts become the "total" flags the encoder below
+// looks for (the row's tokens through each segment), so that an encode in the same call finds every segment's place
+// without waiting: 15 rows of 300,000 to 1,048,576 bp, 32-bit ids, 45 us with the
+// look-back, 18 us with the places known.
+__global__ void __launch_bounds__(256)
+kmer_seg_total_kernel(uint32_t* __restrict__ counts, int64_t n_rows, int n_seg, RowFormat f, int32_t* __restrict__ lengths_out,
+                      int32_t* __restrict__ status) {
+    __shared__ uint32_t s_warp[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int64_t row = blockIdx.x; row < n_rows; row += gridDim.x) {
+        uint32_t carry = 0;                                    // rows hold less than 2^31 bytes and no more tokens
+        for (int s0 = 0; s0 < n_seg; s0 += 256) {
+            const int seg = s0 + tid;
+            uint32_t* const at = counts + (int64_t)seg * n_rows + row;
+            uint32_t x = seg < n_seg ? *at : 0u;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += y;
+            }
+            if (lane == 31) s_warp[warp] = x;
+            __syncthreads();
+            uint32_t before = carry;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) { if (k < warp) before += s_warp[k]; carry += s_warp[k]; }
+            if (seg < n_seg) *at = KSEG_TOTAL | ((before + x) & KSEG_VALUE);     // rows of 2^30 tokens never meet the encoder
+            __syncthreads();
+        }
+        if (tid == 0) {
+            const int64_t n = carry < f.cap_content ? carry : f.cap_content;
+            lengths_out[row] = (int32_t)(n + (f.cls_id >= 0 ? 1 : 0) + (f.sep_id >= 0 ? 1 : 0));
+            if (status && f.clip_is_error && carry > n) atomicOr(status + row, 4);
+        }
+    }
+}
+
 template <typename IdT, int K, bool AFFINE, bool FUSE_MASK>
 __global__ void __launch_bounds__(KW_WARPS * 32, KSEG_BLOCKS_PER_SM)
 kmer_seg_rows_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets, int64_t n_rows,
@@ -768,6 +806,8 @@ kmer_seg_rows_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restric
                      int32_t* __restrict__ lengths_out, const int64_t* __restrict__ out_offsets,
                      int32_t* __restrict__ status, int n_seg, uint32_t* __restrict__ flags,
                      unsigned long long* __restrict__ ticket_counter, int poll_limit, long long withhold) {
+    // ticket_counter == NULL: the flags hold every segment's total (kmer_seg_total_kernel).  Nobody waits for anybody then,
+    // so the segments are dealt round-robin and nothing is published.
     constexpr int NW = (2 * K + 3 + 3) / 4;
     constexpr uint32_t IDX_MASK = (1u << (2 * K)) - 1u;
     constexpr int NCH = KSEG_WINDOWS / 64;
@@ -776,15 +816,20 @@ kmer_seg_rows_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restric
     const int cap = (int)(f.cap_content < 0x7fffffff ? f.cap_content : 0x7fffffff);
     const int64_t mdelta = FUSE_MASK ? (reinterpret_cast<IdT*>(mask) - ids) : 0;
     const int64_t n_tickets = n_rows * (int64_t)n_seg;
+    int64_t t = (int64_t)blockIdx.x * KW_WARPS + (threadIdx.x >> 5) - (int64_t)gridDim.x * KW_WARPS;
     for (;;) {
-        unsigned long long drawn = 0;
-        if (lane == 0) drawn = atomicAdd(ticket_counter, 1ull);
-        const int64_t t = (int64_t)__shfl_sync(0xffffffffu, drawn, 0);
+        if (ticket_counter) {
+            unsigned long long drawn = 0;
+            if (lane == 0) drawn = atomicAdd(ticket_counter, 1ull);
+            t = (int64_t)__shfl_sync(0xffffffffu, drawn, 0);
+        } else {
+            t += (int64_t)gridDim.x * KW_WARPS;
+        }
         if (t >= n_tickets) break;
         const int seg = (int)(t / n_rows);
         const int64_t row = t - (int64_t)seg * n_rows;
         const int64_t off = offsets[row], end = offsets[row + 1];
-        const bool publish = t != (int64_t)withhold;
+        const bool publish = ticket_counter && t != (int64_t)withhold;
 
         const KmerRow<IdT> r = kmer_row_setup<IdT, K>(bytes, off, end, row, total_bytes, f, ids, lengths_in, out_offsets);
         const int64_t w0 = (int64_t)seg * KSEG_WINDOWS;
@@ -796,7 +841,7 @@ kmer_seg_rows_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restric
 
         // the flags of the 32 segments before this one: asked for now, looked at after the decode
         uint32_t look = KSEG_TOTAL;                                              // before the row start: a total of 0
-        if (seg - 1 - lane >= 0) look = *(const volatile uint32_t*)(flags + (int64_t)(seg - 1 - lane) * n_rows + row);
+        if (seg - 1 - lane >= 0 && (ticket_counter || lane == 0)) look = *(const volatile uint32_t*)(flags + (int64_t)(seg - 1 - lane) * n_rows + row);
 
         // ---- 1. decode and count (segments that are not the last of their row hold complete windows only)
         int count = 0;
