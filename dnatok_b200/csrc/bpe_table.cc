@@ -130,6 +130,41 @@ int build_bpe_table(const int32_t* a, const int32_t* b, const int32_t* o, int32_
         if (o[r] >= 32) t->hot_ranks = (uint32_t)r;
     t->byte_tok.resize(256);
     for (int i = 0; i < 256; ++i) t->byte_tok[i] = (uint16_t)byte_ids[i];
+    // The first round in letters: every pair of letters whose rank is below the lowest rank that any of them lets come up.
+    // A word's own bound is no lower (it looks at the pairs that are present), and taking fewer pairs than a round may is
+    // always right.  It asks that no other byte's symbol can merge with any symbol, so that such bytes only separate.
+    t->first.clear();
+    {
+        const char letters[5] = "ACTG";                    // by code
+        std::vector<int32_t> letter_of(n_tokens, -1), bytes_of(n_tokens, 0);
+        for (int i = 0; i < 256; ++i) ++bytes_of[byte_ids[i]];
+        for (int c = 0; c < 4; ++c) letter_of[byte_ids[(unsigned char)letters[c]]] = c;
+        bool ok = safe;
+        uint32_t bound = 0x10000u;
+        uint32_t rank[16];
+        uint16_t made[16] = {0};
+        for (int i = 0; i < 16; ++i) rank[i] = 0xFFFFu;
+        for (int32_t r = 0; r < n && ok; ++r) {
+            if (!bytes_of[a[r]] || !bytes_of[b[r]]) continue;
+            // both operands are symbols: each has to be one letter's and no other byte's
+            const int32_t x = letter_of[a[r]], y = letter_of[b[r]];
+            ok = x >= 0 && y >= 0 && bytes_of[a[r]] == 1 && bytes_of[b[r]] == 1;
+            if (!ok) break;
+            rank[x + 4 * y] = (uint32_t)r;
+            made[x + 4 * y] = (uint16_t)o[r];
+            bound = std::min(bound, (uint32_t)t->future[r]);
+        }
+        if (ok && bound < 0x10000u) {
+            t->first.assign(4096 + 32, 0);
+            for (uint32_t i = 0; i < 4096; ++i) {
+                auto pair = [&](int j) { return rank[(i >> (2 * j)) & 15u]; };
+                for (int j = 0; j < 4; ++j)
+                    t->first[i] |= (uint8_t)((pair(j) < bound ? 1 << j : 0) | (pair(j) > pair(j + 1) ? 16 << j : 0));
+            }
+            for (int i = 0; i < 16; ++i) { t->first[4096 + 2 * i] = (uint8_t)made[i]; t->first[4097 + 2 * i] = (uint8_t)(made[i] >> 8); }
+            t->first_hot = bound <= t->hot_ranks;
+        }
+    }
     t->tok_len.clear();
     if (safe) {                               // operands come before what they create
         t->tok_len.assign(n_tokens, 1);

@@ -26,6 +26,12 @@ struct BpeHostTable {
     bool bytes_hot = false;            // every initial symbol is an id < 32
     std::vector<uint16_t> byte_tok;    // [256] initial symbol of each byte
     std::vector<uint16_t> tok_len;     // [n_tokens] bytes a token stands for, at most 65,535; empty when the table is not batch-safe
+    // The first round of a word of A, C, G, T, looked up letters at a time (empty when it cannot be: see build_bpe_table).
+    // A letter's code is (byte >> 1) & 3.  first[i], i = the codes of six letters, first one lowest: bit j: the pair of letters
+    // j and j + 1 merges in the first round; bit 4 + j: the pair after it ranks better (j < 4).  Behind these 4,096 bytes the
+    // 16 ids (uint16) that the pairs create, at code + 4 * code of the second letter.
+    std::vector<uint8_t> first;
+    bool first_hot = false;            // the first round creates ids below 32 only
     // The same table packed for a kernel that keeps it in shared memory (empty when an id or a displacement does
     // not fit 16 bits): 16-bit displacements [n_tokens + 1], then 32-bit slots (left id << 16) | rank up to the last
     // used one plus one empty slot (larger indices are clamped to it), then one word per rank,

@@ -85,6 +85,7 @@ struct DeviceTables {
     uint16_t* merge_out = nullptr;
     uint64_t* hot = nullptr;
     uint16_t* byte_tok = nullptr;
+    uint8_t* bpe_first = nullptr;    // BPE: the first round in letters (when there is one)
     uint16_t* tok_len = nullptr;     // BPE: bytes per token (when the table is batch-safe)
     int sm_count = 0;
     // host-pipeline staging (grow only)
@@ -155,7 +156,7 @@ int tables_for_current_device(dnatok_handle* h, DeviceTables** out) {
             ~Undo() {
                 if (keep) return;
                 DeviceTables& x = h->dev[dev];
-                void* ptrs[] = {x.lut256, x.start_lut, x.kmer_ids, x.table5, x.exp_off, x.exp_ids, x.disp, x.slots, x.merge_out, x.hot, x.byte_tok, x.tok_len, x.bpe_compact};
+                void* ptrs[] = {x.lut256, x.start_lut, x.kmer_ids, x.table5, x.exp_off, x.exp_ids, x.disp, x.slots, x.merge_out, x.hot, x.byte_tok, x.tok_len, x.bpe_first, x.bpe_compact};
                 for (void* p : ptrs) if (p) cudaFree(p);
                 h->dev.erase(dev);
             }
@@ -177,6 +178,7 @@ int tables_for_current_device(dnatok_handle* h, DeviceTables** out) {
             if ((rc = upload(&d.merge_out, h->bpe.merge_out))) return rc;
             if ((rc = upload(&d.hot, h->bpe.hot))) return rc;
             if ((rc = upload(&d.byte_tok, h->bpe.byte_tok))) return rc;
+            if (!h->bpe.first.empty() && (rc = upload(&d.bpe_first, h->bpe.first))) return rc;
             if (!h->bpe.tok_len.empty() && (rc = upload(&d.tok_len, h->bpe.tok_len))) return rc;
             const BpeLaunchInfo* info;
             if ((rc = bpe_launch_info(dev, &info))) return rc;     // configures every merge kernel once per device
@@ -584,6 +586,7 @@ int run_bpe_merge(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes,
     }
     BpeDeviceTable t{d.disp, reinterpret_cast<const uint2*>(d.slots), d.merge_out, reinterpret_cast<const uint2*>(d.hot),
                      d.byte_tok, h->bpe.batch_safe ? 0 : 1, h->bpe.hot_ranks, h->bpe.bytes_hot ? 1u : 0u, h->bpe.n_tokens,
+                     reinterpret_cast<const uint4*>(d.bpe_first), h->bpe.first_hot ? 1u : 0u,
                      reinterpret_cast<const uint4*>(d.bpe_compact), (uint32_t)h->bpe.compact.size(), h->bpe.compact_slot,
                      h->bpe.compact_info, h->bpe.compact_last};
     // Classes outside the mask are not launched; a row that falls into one is flagged by the classifier.
@@ -1304,7 +1307,7 @@ void dnatok_destroy(dnatok_handle* h) {
         DeviceTables& d = kv.second;
         if (cudaSetDevice(kv.first) != cudaSuccess) continue;
         if (d.stream) cudaStreamSynchronize(d.stream);
-        void* ptrs[] = {d.lut256, d.start_lut, d.table5, d.exp_off, d.exp_ids, d.kmer_ids, d.disp, d.slots, d.merge_out, d.hot, d.byte_tok, d.tok_len, d.bpe_compact, d.st_bytes, d.st_offsets,
+        void* ptrs[] = {d.lut256, d.start_lut, d.table5, d.exp_off, d.exp_ids, d.kmer_ids, d.disp, d.slots, d.merge_out, d.hot, d.byte_tok, d.tok_len, d.bpe_first, d.bpe_compact, d.st_bytes, d.st_offsets,
                         d.st_ids, d.st_mask, d.st_lengths, d.st_status, d.st_out_offsets, d.st_scratch};
         for (void* p : ptrs) if (p) cudaFree(p);
         if (d.stream) cudaStreamDestroy(d.stream);
