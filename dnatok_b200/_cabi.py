@@ -24,6 +24,7 @@ EXPORTS = (
     "dnatok_scan_lengths", "dnatok_encode_host", "dnatok_launch_count", "dnatok_host_copy_bytes",
     "dnatok_encode_bpe_builtin_scratch", "dnatok_set_option", "dnatok_set_row_bytes_hint",
     "dnatok_pack_fasta", "dnatok_embed", "dnatok_create_kmer_table", "dnatok_set_start_lut",
+    "dnatok_row_summary", "dnatok_offset_bounds",
 )
 BUILTIN_SCRATCH_BYTES = 8 << 20
 
@@ -82,6 +83,8 @@ def lib() -> ctypes.CDLL:
     L.dnatok_set_option.argtypes = [c_char_p, c_int64]
     L.dnatok_set_row_bytes_hint.argtypes = [p, c_int64, c_int64]
     L.dnatok_scan_lengths.argtypes = [p, c_int64, p, p]
+    L.dnatok_row_summary.argtypes = [p, p, p, c_int64, p, p, p]
+    L.dnatok_offset_bounds.argtypes = [p, c_int64, p, p]
     L.dnatok_encode_host.argtypes = [p, c_int, p, p, c_int64, POINTER(Format), p, c_int64, p, p, p, p,
                                      POINTER(c_int64)]
     if L.dnatok_version() != 1:

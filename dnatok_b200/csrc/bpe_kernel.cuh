@@ -1058,8 +1058,8 @@ bpe_mixed_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ 
 // common token (a repeat longer than the overlap) sends its word to bpe_long_kernel.
 //
 // One block per word, position-parallel in global memory, left all but a few SMs idle on such batches: 33 words of
-// 40,000 to 400,000 bytes (vocabulary 4,096) took 2,507 us; in windows they take 100 us (merge 75, numbering 8,
-// joins 8, scan 4, copy 5), of which an eighth is work done twice in the overlaps.
+// 40,000 to 400,000 bytes (vocabulary 4,096) took 2,507 us; in windows they take 90 us (merge 67, numbering 8,
+// joins 7, scan 3, copy 5), of which an eighth is work done twice in the overlaps.
 struct BpeWindows {
     int64_t* span;        // [2 * windows] first byte and end of every window in the batch
     int32_t* row_of;      // [windows] index of its word in the list of long words

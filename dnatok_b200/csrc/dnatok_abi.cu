@@ -88,6 +88,9 @@ struct DeviceTables {
     uint8_t* bpe_first = nullptr;    // BPE: the first round in letters (when there is one)
     uint16_t* tok_len = nullptr;     // BPE: bytes per token (when the table is batch-safe)
     int sm_count = 0;
+    // dnatok_row_summary: device words (zero between calls) and the pinned words they end in
+    SummaryWords* summary = nullptr;
+    int64_t* h_summary = nullptr;
     // host-pipeline staging (grow only)
     uint8_t* st_bytes = nullptr;  size_t st_bytes_cap = 0;
     int64_t* st_offsets = nullptr; size_t st_offsets_cap = 0;
@@ -125,6 +128,7 @@ struct dnatok_handle {
     int64_t hint_min_row = 0, hint_max_row = 0;   // caller's bounds on row length in bytes; 0, 0: unknown
     BpeHostTable bpe;
     std::mutex mu;
+    std::mutex summary_mu;
     std::map<int, DeviceTables> dev;
 };
 
@@ -1317,6 +1321,8 @@ void dnatok_destroy(dnatok_handle* h) {
         if (d.st_pipe_rows) cudaFree(d.st_pipe_rows);
         if (d.h_offsets) cudaFreeHost(d.h_offsets);
         if (d.h_rows) cudaFreeHost(d.h_rows);
+        if (d.summary) cudaFree(d.summary);
+        if (d.h_summary) cudaFreeHost(d.h_summary);
     }
     if (!h->dev.empty()) cudaSetDevice(cur);
     delete h;
@@ -1348,6 +1354,45 @@ int dnatok_scan_lengths(const int32_t* d_lengths, int64_t n_rows, int64_t* d_out
     if (!d_lengths || !d_out_offsets || n_rows < 0) return fail(DNATOK_ERR_INVALID, "bad argument");
     scan_lengths_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(d_lengths, n_rows, d_out_offsets);
     LAUNCH_CHECK("scan_lengths_kernel");
+    return DNATOK_OK;
+}
+
+int dnatok_row_summary(dnatok_handle* h, const int32_t* d_lengths, const int32_t* d_status, int64_t n_rows, const int64_t* d_word,
+                       int64_t out[3], dnatok_stream stream) {
+    if (!h || !out || n_rows < 0) return fail(DNATOK_ERR_INVALID, "bad argument");
+    cudaStream_t st = (cudaStream_t)stream;
+    DeviceTables* d;
+    if (int rc = tables_for_current_device(h, &d)) return rc;
+    std::lock_guard<std::mutex> lock(h->summary_mu);          // the words are one call's until it has read them
+    if (!d->summary) {
+        if (!d->h_summary) CUDA_TRY(cudaMallocHost((void**)&d->h_summary, 64));
+        SummaryWords* words = nullptr;
+        CUDA_TRY(cudaMalloc((void**)&words, 256));
+        const cudaError_t e = cudaMemset(words, 0, 256);
+        if (e != cudaSuccess) { cudaFree(words); return fail(DNATOK_ERR_CUDA, "cudaMemset: %s", cudaGetErrorString(e)); }
+        CUDA_TRY(cudaDeviceSynchronize());                    // once per device: the zeroes are there for every stream
+        d->summary = words;
+    }
+    int64_t grid = (n_rows + SUMMARY_PER_BLOCK - 1) / SUMMARY_PER_BLOCK;
+    if (grid > d->sm_count) grid = d->sm_count;
+    if (grid < 1) grid = 1;
+    row_summary_kernel<<<(unsigned)grid, SUMMARY_THREADS, 0, st>>>(d_lengths, d_status, n_rows, d_word, d->summary, d->h_summary);
+    LAUNCH_CHECK("row_summary_kernel");
+    CUDA_TRY(cudaStreamSynchronize(st));
+    for (int i = 0; i < 3; ++i) out[i] = d->h_summary[i];
+    return DNATOK_OK;
+}
+
+int dnatok_offset_bounds(const int64_t* offsets, int64_t n_rows, int64_t* shortest, int64_t* longest) {
+    if (!offsets || n_rows < 0 || !shortest || !longest) return fail(DNATOK_ERR_INVALID, "bad argument");
+    int64_t lo = n_rows ? INT64_MAX : 0, hi = n_rows ? INT64_MIN : 0;
+    for (int64_t i = 0; i < n_rows; ++i) {
+        const int64_t n = offsets[i + 1] - offsets[i];
+        lo = n < lo ? n : lo;
+        hi = n > hi ? n : hi;
+    }
+    *shortest = lo;
+    *longest = hi;
     return DNATOK_OK;
 }
 

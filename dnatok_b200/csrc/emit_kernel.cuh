@@ -455,6 +455,40 @@ __global__ void span_lengths_kernel(const int64_t* __restrict__ offsets, const i
     if (status && f.clip_is_error && n_in > n) atomicOr(status + i, 4);
 }
 
+// What a caller wants to know of a batch's per-row words before it goes on: the largest length, all status bits, and one
+// word copied along (the end of the output offsets).  The last block to finish writes them to host memory and leaves the
+// device words zeroed for the next batch.  One launch and one wait where a reduction and a copy per value took two to four.
+struct SummaryWords { int32_t longest, bits; uint32_t done; };
+constexpr int SUMMARY_THREADS = 256;
+constexpr int SUMMARY_PER_BLOCK = 4096;
+__global__ void __launch_bounds__(SUMMARY_THREADS)
+row_summary_kernel(const int32_t* __restrict__ lengths, const int32_t* __restrict__ status, int64_t n_rows, const int64_t* __restrict__ word,
+                   SummaryWords* __restrict__ w, int64_t* __restrict__ host_out) {
+    __shared__ int32_t s_longest[SUMMARY_THREADS / 32], s_bits[SUMMARY_THREADS / 32];
+    const int tid = threadIdx.x;
+    int32_t longest = 0, bits = 0;
+    for (int64_t i = (int64_t)blockIdx.x * SUMMARY_THREADS + tid; i < n_rows; i += (int64_t)gridDim.x * SUMMARY_THREADS) {
+        if (lengths) longest = max(longest, lengths[i]);
+        if (status) bits |= status[i];
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    bits = (int32_t)__reduce_or_sync(0xffffffffu, (unsigned)bits);
+    if ((tid & 31) == 0) { s_longest[tid >> 5] = longest; s_bits[tid >> 5] = bits; }
+    __syncthreads();
+    if (tid) return;
+    for (int k = 1; k < SUMMARY_THREADS / 32; ++k) { longest = max(longest, s_longest[k]); bits |= s_bits[k]; }
+    atomicMax(&w->longest, longest);
+    atomicOr(&w->bits, bits);
+    __threadfence();
+    if (atomicAdd(&w->done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    host_out[0] = atomicExch(&w->longest, 0);
+    host_out[1] = atomicExch(&w->bits, 0);
+    host_out[2] = word ? *word : 0;
+    atomicExch(&w->done, 0u);
+    __threadfence_system();
+}
+
 // Exclusive scan of int32 lengths into int64 offsets, one block, 4,096 rows per trip: every thread takes four
 // consecutive lengths (one 16-byte load), so a batch of a few thousand rows is one load, one block-wide scan and
 // one round of stores instead of a chain of them.

@@ -107,6 +107,23 @@ class B200Tokenizer:
             return seqs
         return [fn(s) for s in seqs]
 
+    @staticmethod
+    def _row_bounds(host_offsets) -> tuple:
+        """(shortest, longest) row of host offsets."""
+        a = np.ascontiguousarray(host_offsets, dtype=np.int64)
+        out = (ctypes.c_int64 * 2)()
+        at = ctypes.addressof(out)
+        _cabi.check(_cabi.lib().dnatok_offset_bounds(a.ctypes.data, len(a) - 1, at, at + 8))
+        return out[0], out[1]
+
+    def _summary(self, n_rows, stream, lengths=None, status=None, word=0):
+        """(largest length, status bits, *word) once the stream has got here; ``word`` is a device address."""
+        out = (ctypes.c_int64 * 3)()
+        _cabi.check(_cabi.lib().dnatok_row_summary(self.handle.ptr, lengths.data_ptr() if lengths is not None else None,
+                                                   status.data_ptr() if status is not None else None, n_rows, word or None,
+                                                   ctypes.addressof(out), stream))
+        return out[0], out[1], out[2]
+
     # ------------------------------------------------------------------ device-resident path
     def encode_device(self, d_bytes, d_offsets, *, host_offsets: Optional[np.ndarray] = None,
                       padding: Union[bool, str] = "longest", max_length: Optional[int] = None,
@@ -152,8 +169,8 @@ class B200Tokenizer:
         # rows use: large batches of ordinary rows skip the scan of the offsets)
         wants_hint = self.spec.kind == "bpe" or (self.spec.kind == "kmer" and (B < 4096 or total > 32768 * B))
         if wants_hint and host_offsets is not None and B:
-            lens = np.diff(host_offsets)
-            _cabi.check(L.dnatok_set_row_bytes_hint(self.handle.ptr, int(lens.min()), max(int(lens.max()), 1)))
+            shortest, longest = self._row_bounds(host_offsets)
+            _cabi.check(L.dnatok_set_row_bytes_hint(self.handle.ptr, shortest, max(longest, 1)))
         elif self.spec.kind in ("bpe", "kmer"):
             _cabi.check(L.dnatok_set_row_bytes_hint(self.handle.ptr, 0, 0))
         with torch.cuda.device(dev):
@@ -171,6 +188,7 @@ class B200Tokenizer:
             status = torch.empty(max(B, 1), dtype=torch.int32, device=dev)
             args = (self.handle.ptr, ctypes.c_void_p(d_bytes.data_ptr()), ctypes.c_void_p(d_offsets.data_ptr()), B, total)
             res = BatchEncoding()
+            bits = None                            # status bits of the batch, once they are known to be final
 
             if padding is False:
                 fmt = self._format(id_bits=id_bits, mask_bits=0, add_special=add_special_tokens,
@@ -181,7 +199,7 @@ class B200Tokenizer:
                 _cabi.check(L.dnatok_encode(*args, ctypes.byref(fmt), ctypes.c_void_p(ids.data_ptr()), None,
                                             ctypes.c_void_p(lengths.data_ptr()), ctypes.c_void_p(out_off.data_ptr()),
                                             ctypes.c_void_p(status.data_ptr()), sc_ptr, sc_len, stream))
-                n_out = int(out_off[-1].item())
+                _, bits, n_out = self._summary(B, stream, status=status if check and B else None, word=out_off.data_ptr() + 8 * B)
                 res["input_ids"] = ids[:n_out]
                 res["offsets"] = out_off
             else:
@@ -189,16 +207,22 @@ class B200Tokenizer:
                 if padding == "max_length":
                     stride = int(max_length)
                 elif self.spec.kind == "char" and host_offsets is not None:
-                    lens = np.diff(host_offsets)
+                    longest = self._row_bounds(host_offsets)[1]
                     if max_tokens:
-                        lens = np.minimum(lens, max_tokens - ns)
-                    stride = int(lens.max()) + ns if B else 0
+                        longest = min(longest, max_tokens - ns)
+                    stride = longest + ns if B else 0
                 else:
                     fmt0 = self._format(id_bits=id_bits, mask_bits=0, add_special=add_special_tokens,
                                         max_tokens=max_tokens, out_stride=0)
                     _cabi.check(L.dnatok_prepare(*args, ctypes.byref(fmt0), ctypes.c_void_p(lengths.data_ptr()),
                                                  ctypes.c_void_p(status.data_ptr()), sc_ptr, sc_len, stream))
-                    stride = int(lengths[:B].max().item()) if B else 0
+                    stride = 0
+                    if B:
+                        # a BPE row's status is final with its merge (rows padded to the longest are not cut afterwards)
+                        final = check and self.spec.kind == "bpe"
+                        stride, bits, _ = self._summary(B, stream, lengths=lengths, status=status if final else None)
+                        if not final:
+                            bits = None
                     prepared = True
                 fmt = self._format(id_bits=id_bits, mask_bits=mask_bits, add_special=add_special_tokens,
                                    max_tokens=max_tokens, out_stride=stride)
@@ -225,7 +249,10 @@ class B200Tokenizer:
                     res["attention_mask"] = mask
             res["lengths"] = lengths[:B]
             if check and B:
-                self._raise_on_status(status[:B], truncation)
+                if bits is None:
+                    bits = self._summary(B, stream, status=status)[1]
+                if bits:
+                    self._raise_on_status(status[:B], truncation)
         return res
 
     def embed_device(self, d_bytes, d_offsets, weight, *, host_offsets: Optional[np.ndarray] = None,

@@ -192,6 +192,15 @@ int dnatok_encode_bpe_builtin_scratch(dnatok_handle* h, const uint8_t* d_bytes, 
 int dnatok_scan_lengths(const int32_t* d_lengths, int64_t n_rows, int64_t* d_out_offsets,
                         dnatok_stream stream);
 
+/* What a caller needs from a batch's per-row words before it can go on, in one launch and one wait for `stream`:
+ * out[0] = largest of d_lengths, out[1] = all bits of d_status, out[2] = *d_word (for instance the end of the output
+ * offsets).  Each device pointer may be NULL: its value is then 0.  Waits, so not for use under stream capture. */
+int dnatok_row_summary(dnatok_handle* h, const int32_t* d_lengths, const int32_t* d_status, int64_t n_rows,
+                       const int64_t* d_word, int64_t out[3], dnatok_stream stream);
+
+/* Shortest and longest row of HOST offsets (int64[n_rows + 1]); 0, 0 without rows. */
+int dnatok_offset_bounds(const int64_t* offsets, int64_t n_rows, int64_t* shortest, int64_t* longest);
+
 /* Same path with HOST buffers on device `device`: copies bytes and offsets in, runs the kernels,
  * copies ids / mask / lengths / status back and returns when they are in host memory.  Pinned
  * host buffers make the copies asynchronous; pageable ones work.  ids_capacity counts elements

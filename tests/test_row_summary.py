@@ -1,0 +1,53 @@
+"""dnatok_row_summary and dnatok_offset_bounds: what encode_device waits for."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+import helpers as H
+from dnatok_b200 import _cabi
+
+
+@pytest.mark.parametrize("lens,want", [([], (0, 0)), ([5], (5, 5)), ([3, 0, 9, 4], (0, 9))])
+def test_offset_bounds(lens, want):
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    lo, hi = ctypes.c_int64(-1), ctypes.c_int64(-1)
+    _cabi.check(_cabi.lib().dnatok_offset_bounds(_cabi.np_ptr(offs), len(lens), ctypes.byref(lo), ctypes.byref(hi)))
+    assert (lo.value, hi.value) == want
+
+
+@pytest.mark.gpu
+def test_row_summary_sizes_and_threads():
+    """Around the rows of one block, every pointer left out in turn, and from several threads and streams at once."""
+    import torch
+    L = _cabi.lib()
+    handle = _cabi.Handle(H.spec("char"))
+    errors = []
+
+    def work(seed):
+        try:
+            stream = torch.cuda.Stream()
+            rng = np.random.default_rng(seed)
+            for n in [0, 1, 255, 4095, 4096, 4097, 100003]:
+                lens, st = rng.integers(0, 1 << 30, size=n).astype(np.int32), np.zeros(n, np.int32)
+                st[rng.integers(0, n, size=3) if n else []] = [1, 4, 16] if n else []
+                with torch.cuda.stream(stream):
+                    d_l, d_s = torch.from_numpy(lens).cuda(), torch.from_numpy(st).cuda()
+                    word = torch.tensor([seed * 1000003 + n], device="cuda")
+                for a, b, w in [(1, 1, 1), (0, 1, 1), (1, 0, 1), (1, 1, 0)]:
+                    out = (ctypes.c_int64 * 3)()
+                    _cabi.check(L.dnatok_row_summary(handle.ptr, d_l.data_ptr() if a and n else None, d_s.data_ptr() if b and n else None, n,
+                                                     word.data_ptr() if w else None, ctypes.addressof(out), stream.cuda_stream))
+                    assert out[0] == (int(lens.max()) if a and n else 0)
+                    assert out[1] == (int(np.bitwise_or.reduce(st)) if b and n else 0)
+                    assert out[2] == (seed * 1000003 + n if w else 0)
+        except Exception as e:                                  # a thread's assertion has to reach the test
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
