@@ -516,8 +516,9 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
         const int64_t off = offsets[oi];
         const int64_t n64 = here ? offsets[oi + 1] - off : 0;
         int n = (int)n64;                                    // 1 <= n <= T * P by classification (windows: by construction)
-        if (G > 1 && !list && n64 > direct_limit) n = 0;     // flagged at the end
-        if (G == 1 && !WIN && !list && (n64 < 1 || n64 > direct_limit)) {      // direct rows are not vetted: an empty row, or one the hint misstated
+        // direct rows are not vetted: an empty row, one whose offsets decrease (empty as well), or one the hint misstated
+        if (G > 1 && !list && (n64 < 0 || n64 > direct_limit)) n = 0;          // finished with the others of its warp
+        if (G == 1 && !WIN && !list && (n64 < 1 || n64 > direct_limit)) {
             if (g == 0) {
                 counts[row] = 0;
                 bpe_put_length(len_out, row, 0);

@@ -91,3 +91,21 @@ def test_a_row_longer_than_the_hint_is_flagged(longest):
     assert np.array_equal(ln, [0 if over[i] else len(want[i]) for i in range(B)])
     for i in range(0, B, 97):
         assert out[i, :ln[i]].tolist() == ([] if over[i] else want[i].tolist())
+
+
+@pytest.mark.parametrize("rows,lens", [(4737, [100, 250]), (9475, [30, 100]), (19001, [20, 50]), (20003, [20] * 12 + [400])])
+def test_a_row_whose_device_offsets_decrease_comes_out_empty(rows, lens):
+    """Two, four or eight rows per warp as they come, and binned: the host offsets are right, the device's step back."""
+    import torch
+    flat, offs = batch(rows, lens, 90 + rows)
+    bad = offs.copy()
+    at = np.arange(5, rows - 3, rows // 37)
+    bad[at + 1] = bad[at] - 7                                  # row `at` ends before it begins, the next one starts there
+    texts = [flat[bad[i]:bad[i + 1]] if bad[i + 1] > bad[i] else flat[:0] for i in range(rows)]
+    offs2 = np.concatenate([[0], np.cumsum([len(t) for t in texts])]).astype(np.int64)
+    want_ids, want_mask = H.oracle_batch("bpe4096", np.concatenate(texts), offs2, padding="max_length", max_length=60, truncation=True)
+    tok = B200Tokenizer(H.spec("bpe4096"))
+    enc = tok.encode_device(torch.from_numpy(flat).cuda(), torch.from_numpy(bad).cuda(), host_offsets=offs, padding="max_length",
+                            max_length=60, truncation=True)
+    assert np.array_equal(enc["input_ids"].cpu().numpy(), want_ids)
+    assert np.array_equal(enc["attention_mask"].cpu().numpy(), want_mask)
