@@ -696,10 +696,10 @@ int launch_emit(const DeviceTables& d, const SrcT* src, const int64_t* offsets, 
         cfg.numAttrs = g_emit_overlap_launch.load() ? 1 : 0;
         const int32_t* lut = d.lut256;
         if (flat && id_bits == 64)
-            cudaLaunchKernelEx(&cfg, emit_short_kernel<SrcT, int64_t, LUT>, src, offsets, counts, n_rows, lut, rf, (int64_t*)ids, mask,
+            cudaLaunchKernelEx(&cfg, emit_short_kernel<SrcT, int64_t, LUT>, src, total_bytes, offsets, counts, n_rows, lut, rf, (int64_t*)ids, mask,
                                lengths, status);
         else if (flat)
-            cudaLaunchKernelEx(&cfg, emit_short_kernel<SrcT, int32_t, LUT>, src, offsets, counts, n_rows, lut, rf, (int32_t*)ids, mask,
+            cudaLaunchKernelEx(&cfg, emit_short_kernel<SrcT, int32_t, LUT>, src, total_bytes, offsets, counts, n_rows, lut, rf, (int32_t*)ids, mask,
                                lengths, status);
         else if (id_bits == 64)
             cudaLaunchKernelEx(&cfg, emit_padded_kernel<SrcT, int64_t, LUT, EMIT_SPAN>, src, sb, se, offsets, counts, n_rows, lut, rf,

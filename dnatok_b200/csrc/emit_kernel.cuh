@@ -209,8 +209,8 @@ emit_padded_kernel(const SrcT* __restrict__ src, const uint8_t* __restrict__ src
 // 51 / 55; the merged tokens of 65,536 reads of 50 to 300 bp 59 / 16 us.
 template <typename SrcT, typename IdT, bool USE_LUT>
 __global__ void __launch_bounds__(EMIT_THREADS)
-emit_short_kernel(const SrcT* __restrict__ src, const int64_t* __restrict__ offsets, const int32_t* __restrict__ counts, int64_t n_rows,
-                  const int32_t* __restrict__ lut, RowFormat f, IdT* __restrict__ ids, void* __restrict__ mask,
+emit_short_kernel(const SrcT* __restrict__ src, int64_t n_src, const int64_t* __restrict__ offsets, const int32_t* __restrict__ counts,
+                  int64_t n_rows, const int32_t* __restrict__ lut, RowFormat f, IdT* __restrict__ ids, void* __restrict__ mask,
                   int32_t* __restrict__ lengths_out, int32_t* __restrict__ status) {
     constexpr int N = Vec16<IdT>::N;
     asm volatile("griddepcontrol.launch_dependents;");
@@ -227,15 +227,22 @@ emit_short_kernel(const SrcT* __restrict__ src, const int64_t* __restrict__ offs
     const uint32_t step = gridDim.x * EMIT_THREADS, first = blockIdx.x * EMIT_THREADS + threadIdx.x;
     auto elements = [&](uint32_t row, uint32_t* n_in) -> uint32_t {   // content tokens of a row that are kept
         const int64_t n = counts ? (int64_t)counts[row] : offsets[row + 1] - offsets[row];
-        *n_in = (uint32_t)(n < 0x7fffffff ? n : 0x7fffffff);
+        *n_in = (uint32_t)(n < 0 ? 0 : n < 0x7fffffff ? n : 0x7fffffff);          // offsets that decrease make an empty row
         return *n_in < cap ? *n_in : cap;
+    };
+    // The elements of a row that lie in the source buffer; the others are read as 0, as the span kernel does.
+    auto readable = [&](int64_t off, uint32_t n) -> uint32_t {
+        const int64_t room = off < 0 ? 0 : n_src - off;
+        return room < (int64_t)n ? (uint32_t)(room < 0 ? 0 : room) : n;
     };
     const bool ids_aligned = (reinterpret_cast<uintptr_t>(ids) & 15) == 0;
     for (uint32_t g = first * N; g < total; g += step * N) {
         uint32_t row = g / stride, col = g - row * stride, n_in;
         uint32_t n = elements(row, &n_in);
         uint32_t start = (f.pad_left ? stride - n - n_special : 0u) + cls;      // column of the first content token
-        const SrcT* p = src + offsets[row];
+        int64_t off = offsets[row];
+        uint32_t have = readable(off, n);
+        const SrcT* p = src + off;
         IdT vals[N];
 #pragma unroll
         for (int e = 0; e < N; ++e) {
@@ -245,10 +252,13 @@ emit_short_kernel(const SrcT* __restrict__ src, const int64_t* __restrict__ offs
                     col = 0; ++row;
                     n = elements(row, &n_in);
                     start = (f.pad_left ? stride - n - n_special : 0u) + cls;
-                    p = src + offsets[row];
+                    off = offsets[row];
+                    have = readable(off, n);
+                    p = src + off;
                 }
                 const uint32_t t = col - start;                   // wraps below the content
-                if (t < n) v = emit_load<SrcT, USE_LUT>(p + t, s_lut);
+                if (t < have) v = emit_load<SrcT, USE_LUT>(p + t, s_lut);
+                else if (t < n) v = USE_LUT ? s_lut[0] : 0;
                 else if (cls && t == 0xFFFFFFFFu) v = f.cls_id;
                 else if (n_special > cls && t == n) v = f.sep_id;
                 if (col == 0) {

@@ -88,3 +88,40 @@ def test_short_padded_rows(name, left, stride, bits, mask_bits, shift, many):
     assert np.array_equal(got.reshape(-1, stride), want_ids)
     assert np.array_equal(mask.reshape(-1, stride), want_mask)
     assert np.array_equal(lengths, want_mask.sum(1)) and not status.any()
+
+
+@pytest.mark.parametrize("name", ["char", "byte"])
+@pytest.mark.parametrize("left", [False, True])
+@pytest.mark.parametrize("bits,stride", [(32, 17), (64, 40)])
+def test_short_rows_read_the_stated_buffer_only(name, left, bits, stride):
+    """Rows that end behind total_bytes (the letters there belong to the same allocation, but not to the call) read zeros from
+    there on, and a row whose offsets decrease is empty: as the span kernel has it for long rows."""
+    import torch
+    L = _cabi.lib()
+    flat, offs = batch([23, 5, 0, 31, 12, 3, 40, 9] * 30, 8)
+    total = int(offs[-1]) - 30
+    bad = offs.copy()
+    bad[50] = bad[49] - 4
+    seen = flat.copy()
+    seen[total:] = 0
+    texts = [seen[bad[i]:bad[i + 1]] if bad[i + 1] > bad[i] else seen[:0] for i in range(len(bad) - 1)]
+    lens = np.array([len(t) for t in texts])
+    want_ids, want_mask = H.oracle_batch(name, np.concatenate(texts), np.concatenate([[0], np.cumsum(lens)]).astype(np.int64),
+                                         padding="max_length", max_length=stride, truncation=True, pad_left=left,
+                                         id_dtype={32: np.int32, 64: np.int64}[bits], mask_dtype=np.uint8)
+    tok = B200Tokenizer(H.spec(name))
+    B = len(texts)
+    buf = torch.zeros(len(flat) + 4096, dtype=torch.uint8, device="cuda")
+    buf[:len(flat)] = torch.from_numpy(flat).cuda()
+    d_off = torch.from_numpy(bad).cuda()
+    ids = torch.full((B, stride), -7, dtype={32: torch.int32, 64: torch.int64}[bits], device="cuda")
+    mask = torch.full((B, stride), 9, dtype=torch.uint8, device="cuda")
+    lengths, status = (torch.full((B,), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    fmt = _cabi.Format(bits, 8, 1, int(left), stride, stride)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    _cabi.check(L.dnatok_encode(tok.handle.ptr, p(buf), p(d_off), B, total, ctypes.byref(fmt), p(ids), p(mask), p(lengths), None, p(status),
+                                None, 0, None))
+    torch.cuda.synchronize()
+    assert np.array_equal(ids.cpu().numpy(), want_ids)
+    assert np.array_equal(mask.cpu().numpy(), want_mask)
+    assert np.array_equal(lengths.cpu().numpy(), want_mask.sum(1)) and not status.any()
