@@ -321,7 +321,7 @@ kmer_warp_count_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restr
     const int n_special = (f.cls_id >= 0 ? 1 : 0) + (f.sep_id >= 0 ? 1 : 0);
     const int64_t off = offsets[row];
     const int64_t len64 = offsets[row + 1] - off;
-    const int len = (int)(len64 < 0x7fffffff ? len64 : 0x7fffffff);
+    const int len = (int)(len64 < 0 ? 0 : len64 < 0x7fffffff ? len64 : 0x7fffffff);     // offsets that decrease make an empty row
     const int n_win = len / K + (len % K && (!TABLE || t.tail_singles) ? 1 : 0);
     const int cap = (int)(f.cap_content < 0x7fffffff ? f.cap_content : 0x7fffffff);
     const int w_end = n_win <= cap ? n_win : cap + 1;

@@ -214,3 +214,35 @@ def test_clean_window_tables_in_the_row_encoder(k, runs, tail):
                 pad = [0] * (got.shape[1] - len(row))
                 assert got[i].tolist() == (pad + row if side == "left" else row + pad), (side, kw, i)
                 assert mask[i].sum() == len(row) and enc["lengths"][i].item() == len(row)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["kmer6", "table"])
+def test_sizing_of_a_row_whose_device_offsets_decrease(kind):
+    """The host offsets are right, the device's step back: such a row is empty, whatever its (negative) length modulo k."""
+    import helpers as H
+    from dnatok_b200.tokenizer import B200Tokenizer
+    rng = np.random.default_rng(31)
+    lens = rng.integers(40, 90, size=1301)
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    flat = np.frombuffer(b"ACGTN", np.uint8)[rng.choice(5, size=int(offs[-1]), p=[.24, .24, .24, .24, .04])]
+    bad = offs.copy()
+    at = np.arange(3, 1290, 29)
+    bad[at + 1] = bad[at] - np.arange(len(at)) % 14
+    spec = H.spec("kmer6") if kind == "kmer6" else _windows_spec(5, 19, 3)
+    tok = B200Tokenizer(spec)
+    tok.padding_side = "left"
+    texts = [flat[bad[i]:bad[i + 1]].tobytes().decode() if bad[i + 1] > bad[i] else "" for i in range(len(lens))]
+    if kind == "kmer6":
+        o2 = np.concatenate([[0], np.cumsum([len(t) for t in texts])]).astype(np.int64)
+        want = [w.tolist() for w in H.oracle_rows("kmer6", np.frombuffer("".join(texts).encode(), np.uint8), o2)]
+    else:
+        want = [tables.expected_kmer_table_ids(t, spec) for t in texts]
+    enc = tok.encode_device(torch.from_numpy(flat.copy()).cuda(), torch.from_numpy(bad).cuda(), host_offsets=offs, padding="longest",
+                            add_special_tokens=True)
+    got, n = enc["input_ids"].cpu().numpy(), enc["lengths"].cpu().numpy()
+    sp = spec.specials
+    for i, w in enumerate(want):
+        row = ([sp.cls_id] if sp.cls_id >= 0 else []) + w + ([sp.sep_id] if sp.sep_id >= 0 else [])
+        assert n[i] == len(row), i
+        assert got[i].tolist() == [sp.pad_id] * (got.shape[1] - len(row)) + row, i
