@@ -1,6 +1,7 @@
 // C ABI of the library (see include/dnatok_b200.h): handles, table upload, format resolution,
 // kernel launches and the host-buffer pipeline.  No PyTorch, no allocation inside the device
-// entry points other than the one-time table upload per device.
+// entry points other than the one-time table upload per device (and pinned words for more than eight
+// threads at once in dnatok_row_summary).
 #include "../../include/dnatok_b200.h"
 
 #include <atomic>
@@ -88,9 +89,9 @@ struct DeviceTables {
     uint8_t* bpe_first = nullptr;    // BPE: the first round in letters (when there is one)
     uint16_t* tok_len = nullptr;     // BPE: bytes per token (when the table is batch-safe)
     int sm_count = 0;
-    // dnatok_row_summary: device words (zero between calls) and the pinned words they end in
-    SummaryWords* summary = nullptr;
-    int64_t* h_summary = nullptr;
+    // dnatok_row_summary: pinned words, one set per call in flight; summary_chunks: what they were allocated as
+    RowSummary* summary_free = nullptr;
+    RowSummary* summary_chunks = nullptr;
     // host-pipeline staging (grow only)
     uint8_t* st_bytes = nullptr;  size_t st_bytes_cap = 0;
     int64_t* st_offsets = nullptr; size_t st_offsets_cap = 0;
@@ -128,7 +129,7 @@ struct dnatok_handle {
     int64_t hint_min_row = 0, hint_max_row = 0;   // caller's bounds on row length in bytes; 0, 0: unknown
     BpeHostTable bpe;
     std::mutex mu;
-    std::mutex summary_mu;
+    std::mutex summary_mu;             // the lists of dnatok_row_summary's words; never held while a call waits
     std::map<int, DeviceTables> dev;
 };
 
@@ -141,6 +142,25 @@ int upload(T** dst, const std::vector<T>& src) {
     CUDA_TRY(cudaMalloc((void**)dst, src.size() * sizeof(T)));
     CUDA_TRY(cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
     return 0;
+}
+
+// Pinned words for eight more calls of dnatok_row_summary at once.  The first set of a chunk only links the chunks.
+int add_summary_words(DeviceTables* d) {
+    constexpr int SETS = 8;
+    RowSummary* chunk = nullptr;
+    CUDA_TRY(cudaMallocHost((void**)&chunk, (SETS + 1) * sizeof(RowSummary)));
+    chunk[0].next = d->summary_chunks;
+    d->summary_chunks = chunk;
+    for (int i = 1; i <= SETS; ++i) { chunk[i].next = d->summary_free; d->summary_free = chunk + i; }
+    return 0;
+}
+
+void free_summary_words(DeviceTables* d) {
+    while (RowSummary* chunk = d->summary_chunks) {
+        d->summary_chunks = chunk[0].next;
+        cudaFreeHost(chunk);
+    }
+    d->summary_free = nullptr;
 }
 
 struct BpeLaunchInfo;
@@ -162,12 +182,13 @@ int tables_for_current_device(dnatok_handle* h, DeviceTables** out) {
                 DeviceTables& x = h->dev[dev];
                 void* ptrs[] = {x.lut256, x.start_lut, x.kmer_ids, x.table5, x.exp_off, x.exp_ids, x.disp, x.slots, x.merge_out, x.hot, x.byte_tok, x.tok_len, x.bpe_first, x.bpe_compact};
                 for (void* p : ptrs) if (p) cudaFree(p);
+                free_summary_words(&x);
                 h->dev.erase(dev);
             }
         } undo{h, dev, false};
         CUDA_TRY(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
         int rc = upload(&d.lut256, h->lut256);
-        if (rc) return rc;
+        if (rc || (rc = add_summary_words(&d))) return rc;
         if (h->kind == DNATOK_KIND_KMER && !h->kmer_ids.empty() && (rc = upload(&d.kmer_ids, h->kmer_ids))) return rc;
         if (h->kmer_table) {
             if ((rc = upload(&d.table5, h->table5))) return rc;
@@ -1321,8 +1342,7 @@ void dnatok_destroy(dnatok_handle* h) {
         if (d.st_pipe_rows) cudaFree(d.st_pipe_rows);
         if (d.h_offsets) cudaFreeHost(d.h_offsets);
         if (d.h_rows) cudaFreeHost(d.h_rows);
-        if (d.summary) cudaFree(d.summary);
-        if (d.h_summary) cudaFreeHost(d.h_summary);
+        free_summary_words(&d);
     }
     if (!h->dev.empty()) cudaSetDevice(cur);
     delete h;
@@ -1363,23 +1383,35 @@ int dnatok_row_summary(dnatok_handle* h, const int32_t* d_lengths, const int32_t
     cudaStream_t st = (cudaStream_t)stream;
     DeviceTables* d;
     if (int rc = tables_for_current_device(h, &d)) return rc;
-    std::lock_guard<std::mutex> lock(h->summary_mu);          // the words are one call's until it has read them
-    if (!d->summary) {
-        if (!d->h_summary) CUDA_TRY(cudaMallocHost((void**)&d->h_summary, 64));
-        SummaryWords* words = nullptr;
-        CUDA_TRY(cudaMalloc((void**)&words, 256));
-        const cudaError_t e = cudaMemset(words, 0, 256);
-        if (e != cudaSuccess) { cudaFree(words); return fail(DNATOK_ERR_CUDA, "cudaMemset: %s", cudaGetErrorString(e)); }
-        CUDA_TRY(cudaDeviceSynchronize());                    // once per device: the zeroes are there for every stream
-        d->summary = words;
+    struct Words {                                            // this call's until it has read them
+        dnatok_handle* h; DeviceTables* d; RowSummary* w;
+        ~Words() {
+            if (!w) return;
+            std::lock_guard<std::mutex> lock(h->summary_mu);
+            w->next = d->summary_free;
+            d->summary_free = w;
+        }
+    } mine{h, d, nullptr};
+    {
+        std::lock_guard<std::mutex> lock(h->summary_mu);
+        if (!d->summary_free) { if (int rc = add_summary_words(d)) return rc; }
+        mine.w = d->summary_free;
+        d->summary_free = mine.w->next;
     }
     int64_t grid = (n_rows + SUMMARY_PER_BLOCK - 1) / SUMMARY_PER_BLOCK;
-    if (grid > d->sm_count) grid = d->sm_count;
+    if (grid > SUMMARY_BLOCKS) grid = SUMMARY_BLOCKS;
     if (grid < 1) grid = 1;
-    row_summary_kernel<<<(unsigned)grid, SUMMARY_THREADS, 0, st>>>(d_lengths, d_status, n_rows, d_word, d->summary, d->h_summary);
+    row_summary_kernel<<<(unsigned)grid, SUMMARY_THREADS, 0, st>>>(d_lengths, d_status, n_rows, d_word, mine.w);
     LAUNCH_CHECK("row_summary_kernel");
     CUDA_TRY(cudaStreamSynchronize(st));
-    for (int i = 0; i < 3; ++i) out[i] = d->h_summary[i];
+    int32_t longest = 0, bits = 0;
+    for (int64_t i = 0; i < grid; ++i) {
+        longest = mine.w->longest[i] > longest ? mine.w->longest[i] : longest;
+        bits |= mine.w->bits[i];
+    }
+    out[0] = longest;
+    out[1] = bits;
+    out[2] = mine.w->word;
     return DNATOK_OK;
 }
 

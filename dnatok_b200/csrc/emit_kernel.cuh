@@ -466,14 +466,20 @@ __global__ void span_lengths_kernel(const int64_t* __restrict__ offsets, const i
 }
 
 // What a caller wants to know of a batch's per-row words before it goes on: the largest length, all status bits, and one
-// word copied along (the end of the output offsets).  The last block to finish writes them to host memory and leaves the
-// device words zeroed for the next batch.  One launch and one wait where a reduction and a copy per value took two to four.
-struct SummaryWords { int32_t longest, bits; uint32_t done; };
+// word copied along (the end of the output offsets).  Every block leaves its share in the call's own words in pinned host
+// memory, and the host puts the few of them together: nothing is shared between calls, zeroed or allocated on the device.
+// One launch and one wait where a reduction and a copy per value took two to four.
 constexpr int SUMMARY_THREADS = 256;
 constexpr int SUMMARY_PER_BLOCK = 4096;
+constexpr int SUMMARY_BLOCKS = 128;      // most blocks of a launch; above 524,288 rows a block takes more than its 4,096
+struct RowSummary {
+    RowSummary* next;                    // host: list of the words that no call is using
+    int64_t word;
+    int32_t longest[SUMMARY_BLOCKS], bits[SUMMARY_BLOCKS];
+};
 __global__ void __launch_bounds__(SUMMARY_THREADS)
 row_summary_kernel(const int32_t* __restrict__ lengths, const int32_t* __restrict__ status, int64_t n_rows, const int64_t* __restrict__ word,
-                   SummaryWords* __restrict__ w, int64_t* __restrict__ host_out) {
+                   RowSummary* __restrict__ out) {
     __shared__ int32_t s_longest[SUMMARY_THREADS / 32], s_bits[SUMMARY_THREADS / 32];
     const int tid = threadIdx.x;
     int32_t longest = 0, bits = 0;
@@ -487,16 +493,9 @@ row_summary_kernel(const int32_t* __restrict__ lengths, const int32_t* __restric
     __syncthreads();
     if (tid) return;
     for (int k = 1; k < SUMMARY_THREADS / 32; ++k) { longest = max(longest, s_longest[k]); bits |= s_bits[k]; }
-    atomicMax(&w->longest, longest);
-    atomicOr(&w->bits, bits);
-    __threadfence();
-    if (atomicAdd(&w->done, 1u) != gridDim.x - 1) return;
-    __threadfence();
-    host_out[0] = atomicExch(&w->longest, 0);
-    host_out[1] = atomicExch(&w->bits, 0);
-    host_out[2] = word ? *word : 0;
-    atomicExch(&w->done, 0u);
-    __threadfence_system();
+    out->longest[blockIdx.x] = longest;
+    out->bits[blockIdx.x] = bits;
+    if (blockIdx.x == 0) out->word = word ? *word : 0;
 }
 
 // Exclusive scan of int32 lengths into int64 offsets, one block, 4,096 rows per trip: every thread takes four

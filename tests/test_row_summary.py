@@ -51,3 +51,40 @@ def test_row_summary_sizes_and_threads():
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+@pytest.mark.gpu
+def test_a_waiting_call_holds_up_no_other():
+    """While one thread waits for a busy stream, calls on the same handle and another stream return; more of them at once than
+    the words the handle starts with."""
+    import time
+    import torch
+    L = _cabi.lib()
+    handle = _cabi.Handle(H.spec("char"))
+    out = (ctypes.c_int64 * 3)()
+    lens = torch.tensor([3, 9, 4], dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+
+    def summary(stream, out):
+        _cabi.check(L.dnatok_row_summary(handle.ptr, lens.data_ptr(), None, 3, None, ctypes.addressof(out), stream.cuda_stream))
+
+    free = torch.cuda.Stream()
+    summary(free, out)                                          # tables and words are there
+    busy = [torch.cuda.Stream() for _ in range(12)]
+    outs = [(ctypes.c_int64 * 3)() for _ in busy]
+    done = torch.cuda.Event()
+    with torch.cuda.stream(busy[0]):
+        torch.cuda._sleep(1 << 30)                              # about half a second
+        done.record()
+    for s in busy[1:]:
+        s.wait_event(done)
+    threads = [threading.Thread(target=summary, args=(s, o)) for s, o in zip(busy, outs)]
+    for t in threads:
+        t.start()
+    time.sleep(0.1)
+    out[0] = 0
+    summary(free, out)
+    still_busy = not done.query()
+    for t in threads:
+        t.join()
+    assert still_busy and out[0] == 9 and all(o[0] == 9 for o in outs)
