@@ -145,10 +145,13 @@ int upload(T** dst, const std::vector<T>& src) {
 }
 
 // Pinned words for eight more calls of dnatok_row_summary at once.  The first set of a chunk only links the chunks.
-int add_summary_words(DeviceTables* d) {
+// mu (may be NULL): the lock of the lists, not held by the caller nor during the allocation, which may wait for the GPU.
+int add_summary_words(DeviceTables* d, std::mutex* mu) {
     constexpr int SETS = 8;
     RowSummary* chunk = nullptr;
     CUDA_TRY(cudaMallocHost((void**)&chunk, (SETS + 1) * sizeof(RowSummary)));
+    std::unique_lock<std::mutex> lock;
+    if (mu) lock = std::unique_lock<std::mutex>(*mu);
     chunk[0].next = d->summary_chunks;
     d->summary_chunks = chunk;
     for (int i = 1; i <= SETS; ++i) { chunk[i].next = d->summary_free; d->summary_free = chunk + i; }
@@ -188,7 +191,7 @@ int tables_for_current_device(dnatok_handle* h, DeviceTables** out) {
         } undo{h, dev, false};
         CUDA_TRY(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
         int rc = upload(&d.lut256, h->lut256);
-        if (rc || (rc = add_summary_words(&d))) return rc;
+        if (rc || (rc = add_summary_words(&d, nullptr))) return rc;
         if (h->kind == DNATOK_KIND_KMER && !h->kmer_ids.empty() && (rc = upload(&d.kmer_ids, h->kmer_ids))) return rc;
         if (h->kmer_table) {
             if ((rc = upload(&d.table5, h->table5))) return rc;
@@ -1392,11 +1395,13 @@ int dnatok_row_summary(dnatok_handle* h, const int32_t* d_lengths, const int32_t
             d->summary_free = w;
         }
     } mine{h, d, nullptr};
-    {
-        std::lock_guard<std::mutex> lock(h->summary_mu);
-        if (!d->summary_free) { if (int rc = add_summary_words(d)) return rc; }
-        mine.w = d->summary_free;
-        d->summary_free = mine.w->next;
+    while (!mine.w) {
+        {
+            std::lock_guard<std::mutex> lock(h->summary_mu);
+            mine.w = d->summary_free;
+            if (mine.w) d->summary_free = mine.w->next;
+        }
+        if (!mine.w) if (int rc = add_summary_words(d, &h->summary_mu)) return rc;
     }
     int64_t grid = (n_rows + SUMMARY_PER_BLOCK - 1) / SUMMARY_PER_BLOCK;
     if (grid > SUMMARY_BLOCKS) grid = SUMMARY_BLOCKS;
