@@ -450,16 +450,19 @@ __device__ __forceinline__ void bpe_lanes_setup(const BpeLanesShared& sh, const 
 // fits; the n_words rows are taken as they come, and a row longer than direct_limit is flagged and left empty.
 // WIN: the words are the windows of long rows (bpe_window_plan_kernel): offsets holds a (start, end) pair per
 // window, window i's tokens go to out_tok + i * BPE_WIN and its count to counts[i] (-1: it did not converge).
+// SPAN (one team that is the whole block): one word, `span_bytes` bytes from `span_begin`; tokens to out_tok, count to *counts.
 // G (one warp per team only): words a warp works on at once, 32 / G lanes each.  A round's work outside the slots (scans,
 // votes, walk parities) costs a warp the same whatever the word's length, so short words share it.
-template <int W, int BW, int BAR0, int TEAM_BYTES, bool ST = false, bool WIN = false, int G = 1>
+template <int W, int BW, int BAR0, int TEAM_BYTES, bool ST = false, bool WIN = false, int G = 1, bool SPAN = false>
 __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const BpeSmemTable& stab, uint16_t* const sm,
                  const uint8_t* __restrict__ bytes, const int64_t* __restrict__ offsets,
                  const int32_t* __restrict__ list, const int n_words,
                  int32_t* __restrict__ work_counter, const BpeDeviceTable& t,
                  uint16_t* __restrict__ out_tok, int32_t* __restrict__ counts,
-                 int32_t* __restrict__ status, const BpeLengths& len_out, int32_t direct_limit) {
+                 int32_t* __restrict__ status, const BpeLengths& len_out, int32_t direct_limit, int64_t span_begin = 0,
+                 int32_t span_bytes = 0) {
     constexpr int P = BPE_LANE_SLOTS;
+    static_assert(!SPAN || (W == BW && WIN), "a span is a window that the whole block works on");
     static_assert(G == 1 || (W == 1 && !WIN), "only single warps share words");
     constexpr int T = 32 * W / G;                // lanes of a word
     constexpr int L = 32 / G;                    // ... and of them in one warp
@@ -491,7 +494,7 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
     for (;;) {
         int wi;
         if (!work_counter) {
-            wi = first ? (int)blockIdx.x + (int)gridDim.x * (team * G + (G > 1 ? part : 0)) : n_words;
+            wi = !first ? n_words : SPAN ? 0 : (int)blockIdx.x + (int)gridDim.x * (team * G + (G > 1 ? part : 0));
             first = false;
         } else if (G > 1) {
             wi = 0;
@@ -513,8 +516,8 @@ __device__ __forceinline__ void bpe_lanes_body(const BpeLanesShared& sh, const B
         const bool here = G == 1 || wi < n_words;            // the last words may not fill a warp
         const int row = !here ? 0 : !list ? wi : G > 1 ? list[-wi] : list[wi];    // short rows are listed backwards (bpe_classify_kernel)
         const int64_t oi = WIN ? 2 * (int64_t)wi : (int64_t)row;
-        const int64_t off = offsets[oi];
-        const int64_t n64 = here ? offsets[oi + 1] - off : 0;
+        const int64_t off = SPAN ? span_begin : offsets[oi];
+        const int64_t n64 = SPAN ? (int64_t)span_bytes : here ? offsets[oi + 1] - off : 0;
         int n = (int)n64;                                    // 1 <= n <= T * P by classification (windows: by construction)
         // direct rows are not vetted: an empty row, one whose offsets decrease (empty as well), or one the hint misstated
         if (G > 1 && !list && (n64 < 0 || n64 > direct_limit)) n = 0;          // finished with the others of its warp
@@ -1056,11 +1059,14 @@ bpe_mixed_kernel(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ 
 // that crossed one of its borders the merges on either side ran as they run on that pair alone, which would have
 // crossed as well.  (The argument needs no more than the rule itself: lowest rank first, leftmost first.)  Cutting two
 // windows' results at a common token leaves only neighbours that one of the two windows holds.  A border without a
-// common token (a repeat longer than the overlap) sends its word to bpe_long_kernel.
+// common token (a repeat longer than the overlap) is mended by merging more text at once (bpe_mend_word); a word for which
+// that fails goes to bpe_long_kernel.
 //
 // One block per word, position-parallel in global memory, left all but a few SMs idle on such batches: 33 words of
 // 40,000 to 400,000 bytes (vocabulary 4,096) took 2,507 us; in windows they take 90 us (merge 67, numbering 8,
-// joins 7, scan 3, copy 5), of which an eighth is work done twice in the overlaps.
+// joins 7, scan 3, copy 5), of which an eighth is work done twice in the overlaps.  With a homopolymer of 600 bp across one
+// border of every word the call takes 205 us instead of 156, with ten in every word 531 us; 2,640 to 2,740 us when such
+// words were left to bpe_long_kernel.
 struct BpeWindows {
     int64_t* span;        // [2 * windows] first byte and end of every window in the batch
     int32_t* row_of;      // [windows] index of its word in the list of long words
@@ -1186,39 +1192,215 @@ bpe_window_join_kernel(BpeWindows w, const int32_t* __restrict__ n_windows, cons
     }
 }
 
+// The tokens [skip, keep) of a piece that took the places of windows [f, j), dealt to the windows' own places.
+__device__ __forceinline__ void bpe_deal_piece(const BpeWindows& w, int f, int j, int skip, int keep) {
+    for (int k = f + (int)threadIdx.x; k < j; k += blockDim.x) {
+        const int lo = max(skip - (k - f) * BPE_WIN, 0), hi = min(keep - (k - f) * BPE_WIN, BPE_WIN);
+        w.skip[k] = hi > lo ? lo : 0;
+        w.keep[k] = hi > lo ? hi : 0;
+    }
+}
+
+// The borders without a common token of the word in windows [f0, f1), by a block of 32 warps; false: the word is left.
+//
+// A repeat that covers the overlap gives no common token when the windows take it up at different places.  The window
+// before such a border is merged again together with the windows after it, as one piece that is joined as windows are: with
+// the piece or window before it in its first overlap, and with the first window whose overlap with the piece holds a common
+// token.  Three windows are tried, then twelve, then 36, the widest team's 32,768 positions; a repeat beyond that leaves the word
+// to bpe_long_kernel.  A piece takes the windows' own places: it starts where its first window does, and the tokens that
+// begin before the overlap with window j ends are no more than 896 (j - f) + 128, which 1,024 (j - f) places hold.
+constexpr int BPE_MEND_WINDOWS = 36;
+static_assert(BPE_WIN + (BPE_MEND_WINDOWS - 1) * BPE_WIN_STEP <= bpe_class_capacity(BPE_LONG_CLASS - 1), "a piece is one word of the widest team");
+__device__ __forceinline__ bool bpe_mend_word(const BpeLanesShared& sh, uint16_t* const sm, const uint8_t* __restrict__ bytes, const BpeWindows& w,
+                                           const int f0, const int f1, const BpeDeviceTable& t, const uint16_t* __restrict__ tok_len,
+                                           uint16_t* const stage) {
+    constexpr int OV = BPE_WIN_OVERLAP, PER = OV / 32, T = BPE_LONG_WARPS * 32;
+    __shared__ uint16_t s_left[2][OV];                        // overlap before the piece: token that starts there, its index
+    __shared__ int32_t s_n, s_found, s_warp[BPE_LONG_WARPS];
+    uint16_t* const zone_id = sm;                             // [windows of the piece][OV]: the piece's tokens in the overlaps,
+    uint16_t* const zone_at = sm + BPE_MEND_WINDOWS * OV;     // in the merge's buffers once it is done
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int cur = f0, left_f = 0, left_skip = 0, left_end = -1;   // the piece before: first window, tokens skipped, window it joins
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) s_found = INT32_MAX;
+        __syncthreads();
+        for (int k = cur + tid; k < f1; k += T)
+            if (w.keep[k] < 0) { atomicMin(&s_found, k); break; }
+        __syncthreads();
+        const int f = s_found;                                // the next border without a common token
+        if (f == INT32_MAX) return true;
+        if (f == f1 - 1) return false;                        // a window that did not converge
+        const int64_t a = w.span[2 * (int64_t)f];
+        uint16_t* const tok = stage + a;
+        int n, last, hit;
+        for (int m = 3;; m = min(4 * m, BPE_MEND_WINDOWS)) {
+            last = min(f + m, f1) - 1;
+            bpe_lanes_body<BPE_LONG_WARPS, BPE_LONG_WARPS, 1, bpe_team_bytes(BPE_LONG_WARPS), false, true, 1, true>(
+                sh, BpeSmemTable{}, sm, bytes, nullptr, nullptr, 1, nullptr, t, tok, &s_n, nullptr, BpeLengths{}, 0, a,
+                (int32_t)(w.span[2 * (int64_t)last + 1] - a));
+            __syncthreads();
+            n = s_n;
+            if (n < 0) return false;
+            const int zones = last - f + 1;
+            for (int i = tid; i < zones * OV; i += T) zone_id[i] = 0xFFFFu;
+            if (tid == 0) s_found = INT32_MAX;
+            // where the piece's tokens start: every thread takes a run of them
+            const int per = (n + T - 1) / T, q0 = min(tid * per, n), q1 = min(q0 + per, n);
+            int sum = 0;
+            for (int q = q0; q < q1; ++q) sum += (int)__ldg(tok_len + tok[q]);
+            int at = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(BPE_FULL, at, d);
+                if (lane >= d) at += y;
+            }
+            if (lane == 31) s_warp[warp] = at;
+            __syncthreads();
+            at -= sum;
+            for (int k = 0; k < warp; ++k) at += s_warp[k];
+            for (int q = q0; q < q1; ++q) {
+                const uint32_t id = tok[q];
+                const int z = at / BPE_WIN_STEP, p = at - z * BPE_WIN_STEP;
+                if (p < OV && z < zones) { zone_id[z * OV + p] = (uint16_t)id; zone_at[z * OV + p] = (uint16_t)q; }
+                at += (int)__ldg(tok_len + id);
+            }
+            __syncthreads();
+            // the first window that holds one of them at the same place: (window, place, index in the window)
+            for (int z = 1 + warp; z < zones; z += BPE_LONG_WARPS) {
+                const int cb = w.count[f + z];
+                const uint16_t* const tb = w.tok + (int64_t)(f + z) * BPE_WIN;
+                uint32_t id[PER];
+                int start[PER], own = 0;
+#pragma unroll
+                for (int k = 0; k < PER; ++k) {
+                    const int r = PER * lane + k;
+                    id[k] = r < cb ? (uint32_t)tb[r] : 0xFFFFu;
+                    start[k] = own;
+                    own += id[k] != 0xFFFFu ? (int)__ldg(tok_len + id[k]) : OV;
+                }
+                int before = own;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(BPE_FULL, before, d);
+                    if (lane >= d) before += y;
+                }
+                before -= own;
+                uint32_t best = BPE_FULL;
+#pragma unroll
+                for (int k = PER - 1; k >= 0; --k) {
+                    const int p = before + start[k];
+                    if (id[k] != 0xFFFFu && p < OV && zone_id[z * OV + p] == id[k]) best = (uint32_t)((z * OV + p) * OV + PER * lane + k);
+                }
+                best = __reduce_min_sync(BPE_FULL, best);
+                if (lane == 0 && best != BPE_FULL) atomicMin(&s_found, (int)best);
+            }
+            __syncthreads();
+            hit = s_found;
+            if (hit != INT32_MAX || last == f1 - 1) break;
+            if (m == BPE_MEND_WINDOWS) return false;
+            __syncthreads();
+        }
+        // the join before the piece
+        int skip = 0;
+        if (f > f0) {
+            if (left_end != f && warp == 0) {                 // a window, from its end
+                const int ca = w.count[f - 1];
+                const uint16_t* const ta = w.tok + (int64_t)(f - 1) * BPE_WIN;
+                uint32_t id[PER];
+                int end[PER], own = 0;
+#pragma unroll
+                for (int k = 0; k < PER; ++k) s_left[0][lane + 32 * k] = 0xFFFFu;
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < PER; ++k) {
+                    const int r = PER * lane + k;
+                    id[k] = r < ca ? (uint32_t)ta[ca - 1 - r] : 0xFFFFu;
+                    own += id[k] != 0xFFFFu ? (int)__ldg(tok_len + id[k]) : OV;
+                    end[k] = own;                             // bytes from this token's start to the end of the lane's first one
+                }
+                int before = own;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(BPE_FULL, before, d);
+                    if (lane >= d) before += y;
+                }
+                before -= own;
+#pragma unroll
+                for (int k = 0; k < PER; ++k) {
+                    const int p = OV - (before + end[k]);
+                    if (id[k] != 0xFFFFu && p >= 0) { s_left[0][p] = (uint16_t)id[k]; s_left[1][p] = (uint16_t)(ca - 1 - (PER * lane + k)); }
+                }
+            }
+            __syncthreads();
+            if (tid == 0) s_found = INT32_MAX;
+            __syncthreads();
+            if (tid < OV && s_left[0][tid] != 0xFFFFu && s_left[0][tid] == zone_id[tid]) atomicMin(&s_found, tid);
+            __syncthreads();
+            const int p = s_found;
+            if (p == INT32_MAX) return false;
+            skip = (int)zone_at[p] + 1;
+            if (left_end == f) bpe_deal_piece(w, left_f, f, left_skip, (int)s_left[1][p] + 1);
+            else if (tid == 0) w.keep[f - 1] = (int)s_left[1][p] + 1;
+        }
+        const int zp = hit / OV, z = zp / OV;                 // the join after it, or the end of the word
+        const int j = hit == INT32_MAX ? f1 : f + z;
+        uint16_t* const dst = w.tok + (int64_t)f * BPE_WIN;
+        for (int q = tid; q < min(n, (j - f) * BPE_WIN); q += T) dst[q] = tok[q];
+        bpe_deal_piece(w, f, j, skip, hit == INT32_MAX ? n : (int)zone_at[zp] + 1);
+        if (hit == INT32_MAX) return true;
+        if (tid == 0) w.skip[j] = hit % OV + 1;
+        __syncthreads();                                      // s_left has been read
+        if (tid < OV) { s_left[0][tid] = zone_id[z * OV + tid]; s_left[1][tid] = zone_at[z * OV + tid]; }
+        left_f = f; left_skip = skip; left_end = j; cur = j;
+    }
+}
+
 // One block per long word: its token count and the place of every window's tokens, or its entry in the list of words
-// that are left to bpe_long_kernel.
-__global__ void __launch_bounds__(1024)
-bpe_window_scan_kernel(const int32_t* __restrict__ list, const int32_t* __restrict__ list_count, BpeWindows w,
+// that are left to bpe_long_kernel.  Borders without a common token are mended first.
+__global__ void __launch_bounds__(BPE_LONG_WARPS * 32, 1)
+bpe_window_scan_kernel(const uint8_t* __restrict__ bytes, const int32_t* __restrict__ list, const int32_t* __restrict__ list_count,
+                       BpeWindows w, BpeDeviceTable t, const uint16_t* __restrict__ tok_len, uint16_t* __restrict__ out_tok,
                        int32_t* __restrict__ counts, int32_t* __restrict__ status, BpeLengths len_out,
                        int32_t* __restrict__ left_list, int32_t* __restrict__ left_count) {
+    extern __shared__ uint4 bpe_dyn[];
+    BPE_LANES_SHARED(BPE_LONG_WARPS, sh);
     __shared__ int32_t s_warp[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n_words = *list_count;
+    bool ready = false;                                       // the merge's tables are in shared memory
     for (int i = blockIdx.x; i < n_words; i += gridDim.x) {
         const int f = w.first[i], nw = w.first[i + 1] - f;
-        int carry = 0, bad = 0;
-        for (int k0 = 0; k0 < nw; k0 += 1024) {
-            const int k = k0 + tid;
-            int v = 0;
-            if (k < nw) {
-                const int keep = w.keep[f + k];
-                if (keep < 0) bad = 1;
-                v = keep - w.skip[f + k];
-            }
-            int x = v;
+        int carry, bad;
+        for (bool mended = false;; mended = true) {
+            carry = bad = 0;
+            for (int k0 = 0; k0 < nw; k0 += 1024) {
+                const int k = k0 + tid;
+                int v = 0;
+                if (k < nw) {
+                    const int keep = w.keep[f + k];
+                    if (keep < 0) bad = 1;
+                    v = keep - w.skip[f + k];
+                }
+                int x = v;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int y = __shfl_up_sync(BPE_FULL, x, d);
-                if (lane >= d) x += y;
-            }
-            if (lane == 31) s_warp[warp] = x;
-            bad = __syncthreads_or(bad);
-            int before = 0, all = 0;
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(BPE_FULL, x, d);
+                    if (lane >= d) x += y;
+                }
+                if (lane == 31) s_warp[warp] = x;
+                bad = __syncthreads_or(bad);
+                int before = 0, all = 0;
 #pragma unroll
-            for (int q = 0; q < 32; ++q) { if (q < warp) before += s_warp[q]; all += s_warp[q]; }
-            if (k < nw) w.base[f + k] = carry + before + x - v;
-            carry += all;
+                for (int q = 0; q < 32; ++q) { if (q < warp) before += s_warp[q]; all += s_warp[q]; }
+                if (k < nw) w.base[f + k] = carry + before + x - v;
+                carry += all;
+                __syncthreads();
+            }
+            if (!bad || mended) break;
+            if (!ready) bpe_lanes_setup<BPE_LONG_WARPS, false>(sh, t);
+            ready = true;
+            if (!bpe_mend_word(sh, reinterpret_cast<uint16_t*>(bpe_dyn), bytes, w, f, f + nw, t, tok_len, out_tok)) break;
             __syncthreads();
         }
         if (tid == 0) {
@@ -1243,6 +1425,7 @@ bpe_window_write_kernel(const int64_t* __restrict__ offsets, const int32_t* __re
         const int word = w.row_of[i], total = w.total[word];
         if (total < 0) continue;
         const int row = list[word], skip = w.skip[i], m = w.keep[i] - skip, base = w.base[i];
+        if (m == 0) continue;                                 // its tokens are in the pieces around it
         const uint16_t* const src = w.tok + (int64_t)i * BPE_WIN + skip;
         if (len_out.ids) {
             bpe_write_row(len_out, row, total, lane, 32, [&](int q) { return (uint32_t)src[q - base]; }, base, base + m);

@@ -376,7 +376,7 @@ int bpe_launch_info(int dev, const BpeLaunchInfo** out) {
         CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_classify_kernel));
         CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_plan_kernel));
         CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_join_kernel));
-        CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_scan_kernel));
+        CUDA_TRY(cudaFuncSetAttribute(bpe_window_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bpe_team_bytes(BPE_LONG_WARPS)));
         CUDA_TRY(cudaFuncGetAttributes(&fa, bpe_window_write_kernel));
         // ... and the kernels of the output stage, for both id widths
         CUDA_TRY(cudaFuncGetAttributes(&fa, span_lengths_kernel));
@@ -553,7 +553,8 @@ int run_bpe_windows(const DeviceTables& d, const BpeLaunchInfo& li, const BpeDev
     bpe_window_join_kernel<<<grid, BPE_JOIN_WARPS * 32, 0, st>>>(w, n_windows, d.tok_len);
     LAUNCH_CHECK("bpe_window_join_kernel");
     const unsigned word_grid = (unsigned)(n_rows < (int64_t)d.sm_count * 2 ? n_rows : (int64_t)d.sm_count * 2);
-    bpe_window_scan_kernel<<<word_grid, 1024, 0, st>>>(list, list_count, w, s.counts, status, lo, left_list, left_count);
+    bpe_window_scan_kernel<<<word_grid, BPE_LONG_WARPS * 32, bpe_team_bytes(BPE_LONG_WARPS), st>>>(
+        bytes, list, list_count, w, t, d.tok_len, s.tokens, s.counts, status, lo, left_list, left_count);
     LAUNCH_CHECK("bpe_window_scan_kernel");
     bpe_window_write_kernel<<<grid, BPE_JOIN_WARPS * 32, 0, st>>>(offsets, list, w, n_windows, s.tokens, lo);
     LAUNCH_CHECK("bpe_window_write_kernel");
