@@ -807,6 +807,8 @@ void launch_kmer_warp_k(const DeviceTables& d, int32_t affine_base, const uint8_
 // the last segment.
 struct KmerScratch { unsigned long long* tickets; uint32_t* flags; int n_seg; size_t bytes; };
 
+size_t kmer_flag_bytes(int n_seg, int64_t n_rows) { return 256 + (size_t)n_seg * (size_t)n_rows * 4; }
+
 KmerScratch kmer_scratch_layout(const dnatok_handle* h, void* base, int64_t n_rows, int64_t total_bytes) {
     KmerScratch s{};
     if (n_rows <= 0) { s.n_seg = 1; s.bytes = 256; return s; }
@@ -824,7 +826,7 @@ KmerScratch kmer_scratch_layout(const dnatok_handle* h, void* base, int64_t n_ro
     s.n_seg = (int)n_seg;
     s.tickets = (unsigned long long*)base;                       // the ticket counter has the first 256 bytes to itself
     s.flags = (uint32_t*)((uint8_t*)base + 256);
-    s.bytes = 256 + (size_t)n_seg * (size_t)n_rows * 4;
+    s.bytes = kmer_flag_bytes(s.n_seg, n_rows);
     return s;
 }
 
@@ -933,9 +935,9 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
                 int64_t n_rows, int64_t total_bytes, const RowFormat& rf, int id_bits, void* ids, void* mask,
                 const int32_t* lengths_in, int32_t* lengths_out, const int64_t* out_offsets,
                 int32_t* status, void* scratch, size_t scratch_bytes, cudaStream_t st, bool status_unset = false,
-                bool* segments_counted = nullptr) {
-    // segments_counted: set by the sizing pass when the scratch holds every segment's place in its row, read by an encode
-    // that follows in the same call
+                int* segments_counted = nullptr) {
+    // segments_counted: the segments per row whose places the sizing pass left in the scratch (0: none), for an encode that
+    // follows in the same call: it takes the layout from here, since the handle's row-length hint may have changed
     if (n_rows == 0) return 0;
     const int k = h->k;
     // status_unset: the caller left the status words as they were.  The row-per-warp encoder writes every row's word
@@ -988,9 +990,10 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
     if (!COUNT_ONLY && status && scratch && !(reinterpret_cast<uintptr_t>(scratch) & 255) && longest < (1ll << 30) &&
         (few_rows || long_rows || g_kmer_force_segments)) {
         KmerScratch ks = kmer_scratch_layout(h, scratch, n_rows, total_bytes);
+        const bool counted = segments_counted && *segments_counted > 0 && g_kmer_test_withhold.load() < 0;
+        if (counted) { ks.n_seg = *segments_counted; ks.bytes = kmer_flag_bytes(ks.n_seg, n_rows); }
         if (ks.bytes <= scratch_bytes && (ks.n_seg > 1 || g_kmer_force_segments)) {
             if (int rc = zero_now()) return rc;
-            const bool counted = segments_counted && *segments_counted && g_kmer_test_withhold.load() < 0;
             if (counted) ks.tickets = nullptr;
             else CUDA_TRY(cudaMemsetAsync(scratch, 0, ks.bytes, st));
             if (id_bits == 64) launch_kmer_seg<int64_t>(k, d, h->kmer_affine_base, bytes, offsets, n_rows, total_bytes, rf, ids, mask,
@@ -1015,7 +1018,7 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
             kmer_seg_total_kernel<<<(unsigned)(n_rows < 65536 ? n_rows : 65536), 256, 0, st>>>(ks.flags, n_rows, ks.n_seg, rf, lengths_out,
                                                                                            status);
             LAUNCH_CHECK("kmer_seg_total_kernel");
-            if (segments_counted) *segments_counted = true;
+            if (segments_counted) *segments_counted = ks.n_seg;
             return 0;
         }
     }
@@ -1437,7 +1440,7 @@ int dnatok_offset_bounds(const int64_t* offsets, int64_t n_rows, int64_t* shorte
 // segments_counted: see launch_kmer; only dnatok_encode, which owns the scratch between the two steps, passes it.
 static int prepare_rows(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
                         int64_t total_bytes, const dnatok_format* fmt, int32_t* d_lengths, int32_t* d_status,
-                        void* d_scratch, size_t scratch_bytes, dnatok_stream stream, bool* segments_counted) {
+                        void* d_scratch, size_t scratch_bytes, dnatok_stream stream, int* segments_counted) {
     if (int rc = check_batch(h, d_bytes, d_offsets, n_rows, total_bytes)) return rc;
     if (int rc = check_format(fmt, false)) return rc;
     if (!d_lengths) return fail(DNATOK_ERR_INVALID, "d_lengths is NULL");
@@ -1468,7 +1471,7 @@ int dnatok_prepare(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_of
 static int write_rows(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_offsets, int64_t n_rows,
                       int64_t total_bytes, const dnatok_format* fmt, const int32_t* d_lengths,
                       const int64_t* d_out_offsets, void* d_ids, void* d_mask, int32_t* d_status, void* d_scratch,
-                      size_t scratch_bytes, dnatok_stream stream, bool* segments_counted) {
+                      size_t scratch_bytes, dnatok_stream stream, int* segments_counted) {
     if (int rc = check_batch(h, d_bytes, d_offsets, n_rows, total_bytes)) return rc;
     if (int rc = check_format(fmt, false)) return rc;
     if (!d_ids && n_rows) return fail(DNATOK_ERR_INVALID, "d_ids is NULL");
@@ -1533,7 +1536,7 @@ int dnatok_encode(dnatok_handle* h, const uint8_t* d_bytes, const int64_t* d_off
                               (h->kind == DNATOK_KIND_KMER && fmt->pad_left);
     if (need_prepare) {
         if (!d_lengths) return fail(DNATOK_ERR_INVALID, "this format needs d_lengths");
-        bool segments_counted = false;
+        int segments_counted = 0;
         if (int rc = prepare_rows(h, d_bytes, d_offsets, n_rows, total_bytes, fmt, d_lengths, d_status, d_scratch,
                                   scratch_bytes, stream, &segments_counted))
             return rc;
