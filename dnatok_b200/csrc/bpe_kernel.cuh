@@ -78,10 +78,10 @@ struct BpeDeviceTable {
     uint32_t hot_ranks;          // every rank below this creates an id < 32
     uint32_t bytes_hot;          // 1: every initial symbol is an id < 32
     uint32_t filler;             // one past the largest token id: a token whose pairs never merge (disp and slots have room for it)
+    const uint4* first;          // the first round in letters (BpeHostTable::first), NULL when there is none
+    uint32_t first_hot;          // it creates small ids only
     // the table packed for shared memory (NULL when it does not exist): 16-bit displacements, 32-bit slots
     // (left << 16) | rank, one word (F << 16) | created id per rank
-    const uint4* first;          // the first round in letters (BpeHostTable::first), NULL when there is none
-    uint32_t first_hot;
     const uint4* compact;
     uint32_t compact_bytes, compact_slot, compact_info, compact_last;
 };

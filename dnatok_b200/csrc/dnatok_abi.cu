@@ -693,11 +693,11 @@ int launch_emit(const DeviceTables& d, const SrcT* src, const int64_t* offsets, 
     if (rf.out_stride > 0) {
         const uint8_t* sb = reinterpret_cast<const uint8_t*>(src);
         const uint8_t* se = sb + (size_t)total_bytes * sizeof(SrcT);
-        // 32-bit ids on rows of several thousand columns: wider spans, so a trip stores 4 KiB as it does for 64-bit ids
         // Flat for short rows (where the line lies: emit_short_kernel) and for small batches, whose time is the kernel's
         // latency: 200,000 elements take 2.7 us flat and 3.6 us in spans, whatever the rows' length.
         const int64_t elements = n_rows * rf.out_stride;
         const bool flat = elements <= (1 << 18) || (elements < (1ll << 30) && rf.out_stride <= (id_bits == 64 ? 128 : 320));
+        // 32-bit ids on rows of several thousand columns: wider spans, so a trip stores 4 KiB as it does for 64-bit ids
         const bool wide = id_bits == 32 && sizeof(SrcT) == 1 && rf.out_stride >= 4 * EMIT_SPAN_WIDE;
         const int64_t span_cols = wide ? EMIT_SPAN_WIDE : EMIT_SPAN;
         const int64_t spr = (rf.out_stride + span_cols - 1) / span_cols;
@@ -735,7 +735,7 @@ int launch_emit(const DeviceTables& d, const SrcT* src, const int64_t* offsets, 
         else
             cudaLaunchKernelEx(&cfg, emit_padded_kernel<SrcT, int32_t, LUT, EMIT_SPAN>, src, sb, se, offsets, counts, n_rows, lut, rf,
                                (int32_t*)ids, mask, lengths, status, spr, n_spans);
-        LAUNCH_CHECK("emit_padded_kernel");
+        LAUNCH_CHECK(flat ? "emit_short_kernel" : "emit_padded_kernel");
     } else {
         const uint8_t* sb = reinterpret_cast<const uint8_t*>(src);
         const uint8_t* se = sb + (size_t)total_bytes * sizeof(SrcT);
@@ -927,9 +927,6 @@ void launch_kmer_table_rows(int k, const DeviceTables& d, const KmerTable& t, co
 // Otherwise rows of ordinary length go one per warp and batches of very long rows one per block.
 constexpr int64_t KMER_WARP_MAX_AVG_LEN = 32768;
 
-int launch_span_lengths(const int64_t* offsets, const int32_t* counts, int64_t n_rows, const RowFormat& rf,
-                        int32_t* lengths, int32_t* status, cudaStream_t st);
-
 template <bool COUNT_ONLY>
 int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, const int64_t* offsets,
                 int64_t n_rows, int64_t total_bytes, const RowFormat& rf, int id_bits, void* ids, void* mask,
@@ -1050,10 +1047,9 @@ int launch_kmer(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes, c
     return 0;
 }
 
-int launch_span_lengths(const int64_t* offsets, const int32_t* counts, int64_t n_rows, const RowFormat& rf,
-                        int32_t* lengths, int32_t* status, cudaStream_t st) {
+int launch_span_lengths(const int64_t* offsets, int64_t n_rows, const RowFormat& rf, int32_t* lengths, int32_t* status, cudaStream_t st) {
     if (n_rows == 0) return 0;
-    span_lengths_kernel<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(offsets, counts, n_rows, rf, lengths, status);
+    span_lengths_kernel<<<(unsigned)((n_rows + 255) / 256), 256, 0, st>>>(offsets, n_rows, rf, lengths, status);
     LAUNCH_CHECK("span_lengths_kernel");
     return 0;
 }
@@ -1452,7 +1448,7 @@ static int prepare_rows(dnatok_handle* h, const uint8_t* d_bytes, const int64_t*
     if (d_status && n_rows) CUDA_TRY(cudaMemsetAsync(d_status, 0, (size_t)n_rows * 4, st));
     switch (h->kind) {
         case DNATOK_KIND_CHAR:
-            return launch_span_lengths(d_offsets, nullptr, n_rows, rf, d_lengths, d_status, st);
+            return launch_span_lengths(d_offsets, n_rows, rf, d_lengths, d_status, st);
         case DNATOK_KIND_KMER:
             return launch_kmer<true>(h, *d, d_bytes, d_offsets, n_rows, total_bytes, rf, 64, nullptr, nullptr, nullptr, d_lengths,
                                      nullptr, d_status, d_scratch, scratch_bytes, st, false, segments_counted);

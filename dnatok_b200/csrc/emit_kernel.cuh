@@ -223,7 +223,9 @@ emit_short_kernel(const SrcT* __restrict__ src, int64_t n_src, const int64_t* __
     const uint32_t stride = (uint32_t)f.out_stride;
     const uint32_t cls = f.cls_id >= 0 ? 1u : 0u, n_special = cls + (f.sep_id >= 0 ? 1u : 0u);
     const uint32_t cap = (uint32_t)(f.cap_content < (int64_t)stride ? f.cap_content : (int64_t)stride);
-    const uint32_t total = (uint32_t)n_rows * stride;             // below 2^31, see launch_emit
+    // Below 2^30 (launch_emit): the counters below run up to one step of the grid beyond it, at most 19.4 million elements
+    // (148 SMs x 32 blocks x 256 threads x 16 mask bytes), and stay within 32 bits.
+    const uint32_t total = (uint32_t)n_rows * stride;
     const uint32_t step = gridDim.x * EMIT_THREADS, first = blockIdx.x * EMIT_THREADS + threadIdx.x;
     auto elements = [&](uint32_t row, uint32_t* n_in) -> uint32_t {   // content tokens of a row that are kept
         const int64_t n = counts ? (int64_t)counts[row] : offsets[row + 1] - offsets[row];
@@ -453,13 +455,12 @@ __global__ void start_fix_kernel(const uint8_t* __restrict__ bytes, const int64_
     ids[row * f.out_stride + shift + has_cls] = v;
 }
 
-// Row lengths of the one-token-per-element paths (no data is read): min(n, cap) + specials.
-__global__ void span_lengths_kernel(const int64_t* __restrict__ offsets, const int32_t* __restrict__ counts,
-                                    int64_t n_rows, RowFormat f, int32_t* __restrict__ lengths,
+// Row lengths of the one-token-per-character path (no data is read): min(n, cap) + specials.
+__global__ void span_lengths_kernel(const int64_t* __restrict__ offsets, int64_t n_rows, RowFormat f, int32_t* __restrict__ lengths,
                                     int32_t* __restrict__ status) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_rows) return;
-    const int64_t n_in = counts ? (int64_t)counts[i] : offsets[i + 1] - offsets[i];
+    const int64_t n_in = offsets[i + 1] - offsets[i];
     const int64_t n = n_in < f.cap_content ? n_in : f.cap_content;
     lengths[i] = (int32_t)(n + (f.cls_id >= 0 ? 1 : 0) + (f.sep_id >= 0 ? 1 : 0));
     if (status && f.clip_is_error && n_in > n) atomicOr(status + i, 4);

@@ -60,7 +60,11 @@ extern "C" {
 #define DNATOK_KIND_BPE  2
 
 #define DNATOK_BPE_MAX_WORD (1 << 30) /* longest BPE word (bytes): words of up to 32,768 bytes are merged in shared
-                                         memory, longer ones in scratch memory (about 4.5 bytes of scratch per byte) */
+                                         memory, longer ones there in overlapping windows that are joined exactly, or in
+                                         scratch memory where they cannot be (a tandem repeat beyond 32,384 bytes; a merge
+                                         table whose operands are not created by earlier merges; no row length bounds and
+                                         rows of 16 KiB or less on average).  A batch that may hold such a word takes about
+                                         4.5 bytes of scratch per byte */
 
 typedef struct dnatok_handle dnatok_handle;
 typedef void* dnatok_stream;          /* a cudaStream_t */
@@ -194,7 +198,8 @@ int dnatok_scan_lengths(const int32_t* d_lengths, int64_t n_rows, int64_t* d_out
 
 /* What a caller needs from a batch's per-row words before it can go on, in one launch and one wait for `stream`:
  * out[0] = largest of d_lengths, out[1] = all bits of d_status, out[2] = *d_word (for instance the end of the output
- * offsets).  Each device pointer may be NULL: its value is then 0.  Waits, so not for use under stream capture. */
+ * offsets).  Each device pointer may be NULL: its value is then 0.  Waits, so not for use under stream capture.  May be
+ * called on one handle from several threads at once; no call waits for another one's stream. */
 int dnatok_row_summary(dnatok_handle* h, const int32_t* d_lengths, const int32_t* d_status, int64_t n_rows,
                        const int64_t* d_word, int64_t out[3], dnatok_stream stream);
 
