@@ -244,6 +244,9 @@ class B200Tokenizer:
                         _cabi.check(L.dnatok_encode(*args, ctypes.byref(fmt), ids_p, mask_p,
                                                     ctypes.c_void_p(lengths.data_ptr()), None,
                                                     ctypes.c_void_p(status.data_ptr()), sc_ptr, sc_len, stream))
+                elif not prepared:                 # rows without a column: no kernel writes their words
+                    lengths.zero_()
+                    status.zero_()
                 res["input_ids"] = ids
                 if mask is not None:
                     res["attention_mask"] = mask
@@ -297,6 +300,8 @@ class B200Tokenizer:
                                            ctypes.byref(fmt), ctypes.c_void_p(weight.data_ptr()), int(weight.shape[0]),
                                            int(row_bytes), ctypes.c_void_p(out.data_ptr()),
                                            ctypes.c_void_p(lengths.data_ptr()), ctypes.c_void_p(status.data_ptr()), stream))
+        else:
+            lengths.zero_()
         return BatchEncoding(embeddings=out, lengths=lengths[:B])
 
     def _raise_on_status(self, status, truncation: bool) -> None:

@@ -87,3 +87,24 @@ def test_a_waiting_call_holds_up_no_other(waiting):
         t.join()
     assert still_busy or waiting > 8                            # an allocation may wait for the GPU, and others then for it
     assert [o[0] for o in outs] == [9 + k for k in range(waiting + 1)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["byte", "kmer6"])
+def test_empty_rows_padded_to_the_longest(name):
+    """Rows without a column: the words are defined all the same (the memory they come from held others before)."""
+    import torch
+    from dnatok_b200.tokenizer import B200Tokenizer
+    tok = B200Tokenizer(H.spec(name))
+    offs = np.zeros(6, np.int64)
+    d_b, d_o = torch.empty(0, dtype=torch.uint8, device="cuda"), torch.from_numpy(offs).cuda()
+    poison = [torch.full((k,), 5, dtype=torch.int32, device="cuda") for k in (1, 5, 64, 128) for _ in range(8)]
+    del poison
+    for hint in (offs, None):
+        enc = tok.encode_device(d_b, d_o, host_offsets=hint, padding="longest", add_special_tokens=False)
+        assert tuple(enc["input_ids"].shape) == (5, 0) and enc["lengths"].tolist() == [0] * 5
+    if name == "byte":
+        poison = [torch.full((k,), 5, dtype=torch.int32, device="cuda") for k in (1, 5, 64, 128) for _ in range(8)]
+        del poison
+        emb = tok.embed_device(d_b, d_o, torch.zeros((512, 8), device="cuda"), host_offsets=offs, add_special_tokens=False)
+        assert tuple(emb["embeddings"].shape) == (5, 0, 8) and emb["lengths"].tolist() == [0] * 5
