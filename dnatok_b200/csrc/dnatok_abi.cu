@@ -595,8 +595,9 @@ int run_bpe_merge(dnatok_handle* h, const DeviceTables& d, const uint8_t* bytes,
                         ids, rf.mask_bits ? mask : nullptr, rf.out_stride, rf.cls_id, rf.sep_id, rf.pad_id, rf.pad_left,
                         id_bits, rf.mask_bits, status_unset ? 1 : 0};
     // One class only, by the caller's bounds on the row lengths: the rows need no binning, the class's kernel
-    // takes them as they come (and flags a row the bounds misstated).
-    const bool one_class = h->hint_max_row > 0 && (class_mask & (class_mask - 1)) == 0 && !((class_mask >> BPE_LONG_CLASS) & 1u);
+    // takes them as they come (and flags a row the bounds misstated).  No class at all, for a batch of empty rows: the
+    // binning pass writes them.
+    const bool one_class = h->hint_max_row > 0 && class_mask && (class_mask & (class_mask - 1)) == 0 && !((class_mask >> BPE_LONG_CLASS) & 1u);
     // Rows of the first class by the bounds, but shorter on average than their longest: binned by how many fit a warp,
     // where sharing by the longest row gives two at most.  65,536 rows of 50 to 300 bytes, vocabulary 4,096: one row per
     // warp 205 us, two (no binning) 154 us, binned 127 us with the binning pass.

@@ -1101,3 +1101,30 @@ def test_fused_embedding_gather(toks, name, dim, dtype):
     short = weight[:top].contiguous()
     with pytest.raises(_cabi.DnatokError, match="weight matrix"):
         tok.embed_device(d_b, d_o, short, host_offsets=offs, padding="longest")
+
+
+@pytest.mark.parametrize("name", ["bpe4096", "bpe32000"])
+@pytest.mark.parametrize("hint", [True, False])
+def test_bpe_batch_of_empty_rows(name, hint):
+    """No row of the batch has a byte: every layout is written all the same."""
+    from dnatok_b200.tokenizer import B200Tokenizer
+    tok = B200Tokenizer(H.spec(name))
+    offs = np.zeros(6, np.int64)
+    flat = np.zeros(0, np.uint8)
+    d_b, d_o = torch.empty(0, dtype=torch.uint8, device="cuda"), torch.from_numpy(offs).cuda()
+    for special in (True, False):
+        want_ids, want_mask = H.oracle_batch(name, flat, offs, padding="max_length", max_length=7, truncation=True, add_special=special)
+        poison = [torch.full((k,), 5, dtype=torch.int32, device="cuda") for k in (1, 5, 64, 128) for _ in range(8)]
+        out = {k: torch.full((5, 7), 9, dtype=torch.int64, device="cuda") for k in ("input_ids", "attention_mask")}
+        del poison
+        kw = dict(host_offsets=offs if hint else None, add_special_tokens=special)
+        enc = tok.encode_device(d_b, d_o, padding="max_length", max_length=7, truncation=True, out=out, **kw)
+        assert np.array_equal(enc["input_ids"].cpu().numpy(), want_ids) and np.array_equal(enc["attention_mask"].cpu().numpy(), want_mask)
+        assert enc["lengths"].tolist() == [2 * special] * 5
+        enc = tok.encode_device(d_b, d_o, padding="longest", **kw)
+        assert np.array_equal(enc["input_ids"].cpu().numpy(), want_ids[:, :2 * special])
+        enc = tok.encode_device(d_b, d_o, padding=False, **kw)
+        assert enc["offsets"].tolist() == [2 * special * i for i in range(6)]
+        assert np.array_equal(enc["input_ids"].cpu().numpy(), want_ids[:, :2 * special].reshape(-1))
+        host = tok.encode_host((flat, offs), padding="max_length", max_length=7, truncation=True, add_special_tokens=special)
+        assert np.array_equal(host["input_ids"], want_ids) and np.array_equal(host["attention_mask"], want_mask)
